@@ -9,14 +9,13 @@
 //
 //   step k:  (1) factor diagonal block, invert it            (1 CTA)
 //            (2) panel below it  A[i,k] <- A[i,k] * inv_k^T   (row tiles)
-//            (4) X[k, <k]  <- -inv_k * S[k, <k]               (column tiles)
-//            (3) trailing   A[i,j] -= A[i,k] A[j,k]^T         (FFMA GEMM, lower tiles)
+//            (3) X[k, <k]  <- -inv_k * S[k, <k]               (column tiles)
+//   trailing (4) A[i,j] -= A[i,k] A[j,k]^T                    (FFMA GEMM, lower tiles)
 //            (5) S[i>k, <=k] += A[i,k] X[k, <=k]              (FFMA GEMM)
 //
-// (3) and (5) are blocked a second time: four panels form an outer block; a step applies
-// its rank-64 update only to the block's own columns of A and rows of S, and the rest of
-// the matrix gets one update of depth 256 per outer block.  S lives in the not-yet-final
-// part of X.  Everything is fp32 with IEEE division and square root.
+// (4) and (5) run once per outer block of four panels, with depth 256; inside an outer block
+// (2) and (3) apply the block's earlier panels to their tiles themselves.  S lives in the
+// not-yet-final part of X.  Everything is fp32 with IEEE division and square root.
 #include "common.cuh"
 #include "sgemm.cuh"
 #include <algorithm>
@@ -27,7 +26,6 @@ namespace jgq {
 
 constexpr int CB = 64;          // panel width
 constexpr int COB = 4;          // panels per outer block (deferred updates of depth 256)
-constexpr int CPAD = CB + 1;
 
 // ---- (0) diagonal statistics: dead features, damping increment ----------------
 __global__ void __launch_bounds__(1024)
@@ -78,226 +76,409 @@ __global__ void zero_dead_rows_kernel(float* __restrict__ W, int K, int64_t N,
     W[(int64_t)r * N + c] = 0.f;
 }
 
-// ---- one panel step: factor + invert the 64x64 diagonal block (one CTA), then the step's tiles ----
-// The diagonal block is factored by a single CTA and its inverse handed to the tile kernel through
-// X; the tile kernel is launched with programmatic stream serialization, so its CTAs are already
-// placed (and have fetched their own tiles) when the diagonal kernel ends.  The 64x64 block is
-// processed in 16-wide sub-blocks: a single warp factors and inverts a 16x16 block with register
-// rows and shuffles (no block-wide barrier inside), the rest is small shared-memory products.
+// ---- one panel step: two launches, chained with programmatic stream serialization ----------------
+// What bounds the sweep below K of a few thousand is the latency of this chain, K / 64 times in a row, so
+// both kernels are built for it: one pass over the pivots of a diagonal block gives the factor and its inverse,
+// and everything of the tile kernel that does not need the diagonal block - the updates with the outer
+// block's earlier panels - runs beside the diagonal kernel.  Every element's products are summed in the same
+// order as in a plain blocked sweep (increasing contraction index inside a panel, panel by panel), so that
+// neither the tiling nor the fusion shows in the result.  Measured
+// per panel at K = 768 (serialised): diagonal 38 -> 13.4 us, tiles 19.4 -> 16.5 us with the rank-64 updates in them,
+// whose own launch (24 us) is gone; the whole stage 757 -> 315 us at K = 768, 3407 -> 1690 at 3072, 5190 -> 2917 at 4096.
 
-// 16x16 Cholesky + inverse of the lower-triangular factor, one warp; lanes 16..31 mirror 0..15.
-__device__ __forceinline__ bool leaf16(float (*a)[CPAD], float (*inv)[CPAD], const int c0) {
-  const unsigned full = 0xffffffffu;
-  const int lane = threadIdx.x & 31, r = lane & 15;
-  float v[16], x[16];
-#pragma unroll
-  for (int j = 0; j < 16; ++j) v[j] = (j <= r) ? a[c0 + r][c0 + j] : 0.f;
-  bool notpd = false;
-#pragma unroll
-  for (int k = 0; k < 16; ++k) {
-    const float akk = __shfl_sync(full, v[k], k);
-    notpd |= !(akk > 0.f);
-    const float d = __fsqrt_rn(akk);
-    const float lk = (r == k) ? d : __fdiv_rn(v[k], d);      // l[r][k], meaningful for r >= k
-    v[k] = lk;
-#pragma unroll
-    for (int j = k + 1; j < 16; ++j) {
-      const float ljk = __shfl_sync(full, lk, j);             // l[j][k]
-      v[j] = fmaf(-lk, ljk, v[j]);                            // a[r][j] -= l[r][k] l[j][k]   (r >= j)
-    }
-  }
-  // column r of the inverse by forward substitution; row i of L lives in lane i
-#pragma unroll
-  for (int i = 0; i < 16; ++i) {
-    const float lii = __shfl_sync(full, v[i], i);
-    float sum = 0.f;
-#pragma unroll
-    for (int m = 0; m < i; ++m) {
-      const float lim = __shfl_sync(full, v[m], i);
-      sum = fmaf(lim, x[m], sum);
-    }
-    x[i] = (i == r) ? __fdiv_rn(1.f, lii) : ((i > r) ? __fdiv_rn(-sum, lii) : 0.f);
-  }
-  if (lane < 16) {
-#pragma unroll
-    for (int j = 0; j < 16; ++j) {
-      if (j <= r) a[c0 + r][c0 + j] = v[j];
-      inv[c0 + j][c0 + r] = x[j];
-    }
-  }
-  return __any_sync(full, notpd);
+constexpr int CS = CB + 4;      // row stride of the shared 64 x 64 tiles: 16-byte rows, eight rows on 32 banks
+
+// d = sqrt(a) and y = 1 / d, both rounded to nearest, for a in [2^-96, 2^96]: Goldschmidt iterations on the
+// hardware's reciprocal root with the residual corrections of Markstein (IBM J. R&D 34, 1990).  Checked
+// against the IEEE operations over every mantissa and both exponent parities: d always, y but for d's largest mantissa.  About 70 cycles for the
+// pair; an IEEE root takes 55, and each division by it 50 more where divide_by takes 20.
+__device__ __forceinline__ void root_and_reciprocal(float a, float& d, float& y) {
+  float h, g, e;
+  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(a));
+  g = a * y;
+  h = 0.5f * y;
+  e = fmaf(-h, g, 0.5f);
+  g = fmaf(g, e, g);
+  h = fmaf(h, e, h);
+  e = fmaf(-g, g, a);
+  d = fmaf(e, h, g);
+  y = h + h;
+  e = fmaf(-d, y, 1.f);
+  y = fmaf(y, e, y);
+  e = fmaf(-d, y, 1.f);
+  y = fmaf(y, e, y);
+}
+// num / d rounded to nearest, given y = 1 / d rounded to nearest (Markstein's theorem: a quotient within one unit
+// in the last place, corrected once more with the exact residual).  The residual must stay above the subnormals:
+// `ok` is cleared unless |num| is zero or in [2^-90, 2^90].
+__device__ __forceinline__ float divide_by(float num, float d, float y, bool& ok) {
+  float q = num * y;
+  float e = fmaf(-d, q, num);
+  q = fmaf(e, y, q);
+  e = fmaf(-d, q, num);
+  q = fmaf(e, y, q);
+  const float m = fabsf(num);
+  ok &= (m >= 8.0779356694631609e-28f && m <= 1.2379400392853803e27f) || m == 0.f;
+  return m == 0.f ? num : q;
 }
 
+// Cholesky factor of the 16 x 16 block at (c0, c0) of `a` (lower triangle significant) and its inverse, one
+// warp, one pass.  Lane r < 16 holds row r of the block, lane 16 + c the running sums of column c of the
+// forward substitution L X = I.  Pivot k: everybody divides its element k by the pivot's root (column k of L in
+// the one half, row k of the inverse in the other), and the products with column k of L go to both the block and
+// the sums.  The chain from pivot to pivot is root, quotient, one shuffle and one multiply-add: every lane follows
+// the whole diagonal (dg), element k + 1 of column k comes by shuffle, the others (needed a pivot later) through
+// shared memory; their products are put off until the next pivot's root is under way.  A warp is alone with this
+// chain, so the loop has no branch that would keep its instructions from overlapping: kFast = false is the same
+// elimination with the IEEE operations, for the blocks whose values leave the range of the fast ones (returns
+// false then; `iv` is written only on success).
+template <bool kFast>
+__device__ __forceinline__ bool leaf16(const float (*a)[CS], float (*iv)[20], float* col, const int c0, bool& notpd) {
+  const unsigned full = 0xffffffffu;
+  const int lane = threadIdx.x & 31, r = lane & 15;
+  const bool upper = lane >= 16;                  // the half that builds the inverse
+  float v[16], dg[16], l[16], tp = 0.f;
+#pragma unroll
+  for (int j = 0; j < 16; ++j) {
+    v[j] = (!upper && j <= r) ? a[c0 + r][c0 + j] : 0.f;
+    dg[j] = a[c0 + j][c0 + j];
+    l[j] = 0.f;
+  }
+  bool ok = true;
+  notpd = false;
+#pragma unroll
+  for (int k = 0; k < 16; ++k) {
+    const float akk = dg[k];
+    float d, y = 0.f;
+    if (kFast) {
+      root_and_reciprocal(akk, d, y);
+      ok &= akk >= 1.2621774483536189e-29f && akk <= 7.9228162514264338e28f &&
+            (__float_as_uint(d) & 0x7fffffu) != 0x7fffffu;      // the one mantissa whose reciprocal the iteration misses
+    } else {
+      d = __fsqrt_rn(akk);
+    }
+    notpd |= !(akk > 0.f);
+    // products with column k - 1, from row k + 1 on
+    if (k > 0) {
+#pragma unroll
+      for (int j = k + 1; j < 16; ++j) {
+        dg[j] = fmaf(l[j], -l[j], dg[j]);
+        v[j] = fmaf(l[j], tp, v[j]);
+      }
+    }
+    const float num = upper ? (r == k ? 1.f : -v[k]) : v[k];
+    float q = kFast ? divide_by(num, d, y, ok) : __fdiv_rn(num, d);
+    if (!upper && r == k) q = d;
+    if (upper && r > k) q = 0.f;
+    const float t = upper ? q : -q;
+    v[k] = q;
+    tp = t;
+    if (k < 15) {
+      const float lnext = __shfl_sync(full, q, k + 1);
+      float* cb = col + 16 * (k & 1);
+      if (!upper) cb[r] = q;
+      dg[k + 1] = fmaf(lnext, -lnext, dg[k + 1]);
+      v[k + 1] = fmaf(lnext, t, v[k + 1]);
+      __syncwarp();
+#pragma unroll
+      for (int j4 = 0; j4 < 16; j4 += 4)
+        if (j4 + 3 >= k + 2) {
+          const float4 l4 = *reinterpret_cast<const float4*>(cb + j4);
+          l[j4] = l4.x; l[j4 + 1] = l4.y; l[j4 + 2] = l4.z; l[j4 + 3] = l4.w;
+        }
+    }
+  }
+  if (kFast && !__all_sync(full, ok)) return false;
+  if (upper) {
+#pragma unroll
+    for (int i = 0; i < 16; ++i) iv[i][r] = v[i];
+  }
+  return true;
+}
+
+// 64 x 64 tile at (row, col) of a K-stride matrix into registers: thread t holds four consecutive columns
+// 4 (t % 16) of rows t / 16 + 16 q; zeros from row_lim / col_lim on.  `vec`: 16-byte loads are legal.
+__device__ __forceinline__ void tile_fetch(float4 (&v)[4], const float* __restrict__ P, int K, int row, int col,
+                                           int row_lim, int col_lim, bool vec) {
+  const int t = threadIdx.x, j = col + 4 * (t & 15);
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    const int i = row + (t >> 4) + 16 * q;
+    const float* src = P + (int64_t)i * K + j;
+    v[q] = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (i < row_lim) {
+      if (vec && j + 3 < col_lim) v[q] = *reinterpret_cast<const float4*>(src);
+      else {
+        if (j < col_lim) v[q].x = src[0];
+        if (j + 1 < col_lim) v[q].y = src[1];
+        if (j + 2 < col_lim) v[q].z = src[2];
+        if (j + 3 < col_lim) v[q].w = src[3];
+      }
+    }
+  }
+}
+__device__ __forceinline__ void tile_put(float (*S)[CS], const float4 (&v)[4]) {
+  const int t = threadIdx.x;
+#pragma unroll
+  for (int q = 0; q < 4; ++q) *reinterpret_cast<float4*>(&S[(t >> 4) + 16 * q][4 * (t & 15)]) = v[q];
+}
+
+// Inverse of the Cholesky factor of diagonal block kb, written to X; the factor itself is not needed again.
+// Sixteen columns at a time: leaf16 inverts the pivot block (iv); the rows below become P = A iv^T and the
+// pivot rows of the inverse X = -iv T, T being the sums P X of the earlier steps; then the rows below take
+// A -= P P^T and T += P X.  R holds the right factors of both updates side by side (P^T, then the pivot rows
+// of X), so that they are one loop.  Warp 0 brings the next pivot block up to date and goes on with it while
+// the other warps finish the update.
 __global__ void __launch_bounds__(256)
-chol_diag_kernel(const float* __restrict__ A, float* __restrict__ X, int K, int kb,
+chol_diag_kernel(const float* __restrict__ A, float* __restrict__ X, int K, int kb, int vec,
                  int32_t* __restrict__ status) {
-  __shared__ float a[CB][CPAD];
-  __shared__ float inv[CB][CPAD];
+  __shared__ __align__(16) float a[CB][CS];
+  __shared__ __align__(16) float x[CB][CS];        // T
+  __shared__ __align__(16) float R[16][2 * CB + 4];
+  __shared__ __align__(16) float P[CB - 16][20];   // from row 16 on
+  __shared__ __align__(16) float iv[16][20];
+  __shared__ __align__(16) float col[32];
   const int r0 = kb * CB;
   const int nb = min(CB, K - r0);
   const int tid = threadIdx.x, warp = tid >> 5;
-  for (int idx = tid; idx < CB * CB; idx += 256) {
-    const int i = idx / CB, j = idx % CB;
-    float v = 0.f;
-    if (i < nb && j <= i) v = A[(int64_t)(r0 + i) * K + r0 + j];
-    else if (i >= nb && i == j) v = 1.f;            // identity padding of a partial last block
-    a[i][j] = v;
-    inv[i][j] = 0.f;
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  // The tile kernel of this step may be scheduled from here on: all it reads before its own wait was
+  // complete when this wait returned.
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  {
+    float4 v[4];
+    tile_fetch(v, A, K, r0, r0, K, K, vec != 0);
+    tile_put(a, v);
+#pragma unroll
+    for (int q = 0; q < 4; ++q) v[q] = make_float4(0.f, 0.f, 0.f, 0.f);
+    tile_put(x, v);
   }
   __syncthreads();
+  if (nb < CB) {
+    if (tid >= nb && tid < CB) a[tid][tid] = 1.f;   // identity padding of a partial last block
+    __syncthreads();
+  }
 
-  // ---- blocked (16) right-looking Cholesky of the 64x64 block, diagonal sub-blocks inverted ----
+  // one item = 4 columns of one row of the update of step c0 / 16: rows / 4 items per row for A, (c0 + 16) / 4 for T
+  auto update = [&](int c0, int i, int qd) {
+    const int rows = CB - 16 - c0, b0 = c0 + 16;
+    const bool ina = qd < rows / 4;
+    const int cl = ina ? b0 + 4 * qd : 4 * (qd - rows / 4);
+    const int rc = ina ? cl : CB + cl;
+    float4* dst = reinterpret_cast<float4*>(ina ? &a[i][cl] : &x[i][cl]);
+    const float4 old = *dst;
+    float4 acc = ina ? make_float4(0.f, 0.f, 0.f, 0.f) : old;
+#pragma unroll
+    for (int m4 = 0; m4 < 16; m4 += 4) {
+      const float4 pm = *reinterpret_cast<const float4*>(&P[i - 16][m4]);
+      const float pj[4] = {pm.x, pm.y, pm.z, pm.w};
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const float4 w = *reinterpret_cast<const float4*>(&R[m4 + u][rc]);
+        acc.x = fmaf(pj[u], w.x, acc.x); acc.y = fmaf(pj[u], w.y, acc.y);
+        acc.z = fmaf(pj[u], w.z, acc.z); acc.w = fmaf(pj[u], w.w, acc.w);
+      }
+    }
+    if (ina) acc = make_float4(old.x - acc.x, old.y - acc.y, old.z - acc.z, old.w - acc.w);
+    *dst = acc;
+  };
+
+#pragma unroll 1
   for (int s = 0; s < 4; ++s) {
-    const int c0 = 16 * s;
+    const int c0 = 16 * s, rows = CB - 16 - c0, b0 = c0 + 16;
     if (warp == 0) {
-      const bool bad = leaf16(a, inv, c0);
+      if (s > 0) {
+        // the pivot block itself: its 16 columns are the first four items of a row
+#pragma unroll
+        for (int h = 0; h < 2; ++h) update(c0 - 16, c0 + ((tid + 32 * h) >> 2), tid & 3);
+        __syncwarp();
+      }
+      bool bad;
+      if (!leaf16<true>(a, iv, col, c0, bad)) leaf16<false>(a, iv, col, c0, bad);
       if (bad && tid == 0) atomicOr(status, JGQ_STATUS_NOT_PD);
+    } else if (s > 0) {
+      for (int item = tid - 32; item < (rows + 16) * 16; item += 224) {
+        const int i = c0 + (item >> 4), qd = item & 15;
+        if (i >= b0 || qd >= 4) update(c0 - 16, i, qd);
+      }
     }
     __syncthreads();
-    const int rows = CB - (c0 + 16);
-    if (rows > 0) {
-      float pv[3];
+    // 48 x 16 elements, three per thread: first the rows below (P), then the earlier columns of the pivot rows of X
 #pragma unroll
-      for (int t = 0; t < 3; ++t) {
-        const int idx = tid + 256 * t;
-        pv[t] = 0.f;
-        if (idx < rows * 16) {
-          const int i = c0 + 16 + idx / 16, c = idx % 16;
-          float sum = 0.f;
-          for (int m = 0; m <= c; ++m) sum = fmaf(a[i][c0 + m], inv[c0 + c][c0 + m], sum);
-          pv[t] = sum;
+    for (int t = 0; t < 3; ++t) {
+      const int u = tid / 16 + 16 * t, c = tid % 16;       // u < rows: row b0 + u, column c of P
+      float sum = 0.f;
+      if (u < rows) {
+        const int i = b0 + u;
+#pragma unroll
+        for (int m = 0; m < 16; m += 4) {
+          const float4 p4 = *reinterpret_cast<const float4*>(&a[i][c0 + m]);
+          const float4 w = *reinterpret_cast<const float4*>(&iv[c][m]);
+          sum = fmaf(p4.x, w.x, sum); sum = fmaf(p4.y, w.y, sum); sum = fmaf(p4.z, w.z, sum); sum = fmaf(p4.w, w.w, sum);
         }
-      }
-      __syncthreads();
+        P[i - 16][c] = sum;
+        R[c][i] = sum;
+      } else {
+        const int cc = u - rows, rr = c;                    // element (rr, cc) of the pivot rows, cc < c0
 #pragma unroll
-      for (int t = 0; t < 3; ++t) {
-        const int idx = tid + 256 * t;
-        if (idx < rows * 16) a[c0 + 16 + idx / 16][c0 + idx % 16] = pv[t];
+        for (int m = 0; m < 16; ++m) sum = fmaf(iv[rr][m], x[c0 + m][cc], sum);
+        R[rr][CB + cc] = -sum;
+        if (c0 + rr < nb) X[(int64_t)(r0 + c0 + rr) * K + r0 + cc] = -sum;
       }
-      __syncthreads();
-      for (int idx = tid; idx < rows * rows; idx += 256) {
-        const int i = c0 + 16 + idx / rows, j = c0 + 16 + idx % rows;
-        if (j <= i) {
-          float sum = 0.f;
-#pragma unroll
-          for (int m = 0; m < 16; ++m) sum = fmaf(a[i][c0 + m], a[j][c0 + m], sum);
-          a[i][j] -= sum;
-        }
-      }
-      __syncthreads();
     }
-  }
-
-  // ---- assemble the inverse from its 16x16 diagonal blocks, one block diagonal at a time ----
-  {
-    const int rr = tid / 16, cc = tid % 16;
-    for (int d = 1; d < 4; ++d) {
-      float tv[3];
-#pragma unroll
-      for (int bi = 0; bi < 3; ++bi) {
-        const int i = d + bi, j = bi;           // block (i, j), i - j == d
-        tv[bi] = 0.f;
-        if (i < 4) {
-          float sum = 0.f;
-          for (int m = j; m < i; ++m)
-#pragma unroll
-            for (int q = 0; q < 16; ++q) sum = fmaf(a[16 * i + rr][16 * m + q], inv[16 * m + q][16 * j + cc], sum);
-          tv[bi] = sum;
-        }
-      }
-      __syncthreads();
-#pragma unroll
-      for (int bi = 0; bi < 3; ++bi)
-        if (d + bi < 4) inv[16 * (d + bi) + rr][16 * bi + cc] = tv[bi];
-      __syncthreads();
-#pragma unroll
-      for (int bi = 0; bi < 3; ++bi) {
-        const int i = d + bi, j = bi;
-        if (i < 4) {
-          float sum = 0.f;
-          for (int q = 0; q <= rr; ++q) sum = fmaf(inv[16 * i + rr][16 * i + q], inv[16 * i + q][16 * j + cc], sum);
-          tv[bi] = -sum;
-        }
-      }
-      __syncthreads();
-#pragma unroll
-      for (int bi = 0; bi < 3; ++bi)
-        if (d + bi < 4) inv[16 * (d + bi) + rr][16 * bi + cc] = tv[bi];
-      __syncthreads();
+    {
+      const int rr = tid / 16, c = tid % 16;
+      const float v = iv[rr][c];
+      R[rr][CB + c0 + c] = v;
+      if (c0 + rr < nb && c0 + c < nb) X[(int64_t)(r0 + c0 + rr) * K + r0 + c0 + c] = v;
     }
-  }
-
-  // The tile kernel of this step may be scheduled from here on; it still waits for this grid to end.
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-  // The inverse of the diagonal block is part of the result X, and what the tiles of this step read.
-  // The factor itself is not written back: nothing reads it after this step.
-  for (int idx = tid; idx < nb * nb; idx += 256) {
-    const int i = idx / nb, j = idx % nb;
-    X[(int64_t)(r0 + i) * K + r0 + j] = inv[i][j];
+    __syncthreads();
   }
 }
 
-// One 64x64 tile of a panel step per CTA: (2) a tile of the panel below the diagonal block, or (4) a tile
-// of row block kb of the inverse.  Launched with programmatic stream serialization behind chol_diag_kernel:
-// the CTA fetches its own tile (complete before the diagonal kernel began) and only then waits for the
-// diagonal kernel's result.
+// acc[i][j] += sum_m U[ty + 16 i][m] V[tx + 16 j][m]
+__device__ __forceinline__ void tile_mul_nt(float (&acc)[4][4], const float (*U)[CS], const float (*V)[CS]) {
+  const int ty = threadIdx.x >> 4, tx = threadIdx.x & 15;
+#pragma unroll 4
+  for (int m = 0; m < CB; m += 4) {
+    float4 u[4], w[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      u[i] = *reinterpret_cast<const float4*>(&U[ty + 16 * i][m]);
+      w[i] = *reinterpret_cast<const float4*>(&V[tx + 16 * i][m]);
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        acc[i][j] = fmaf(u[i].x, w[j].x, acc[i][j]); acc[i][j] = fmaf(u[i].y, w[j].y, acc[i][j]);
+        acc[i][j] = fmaf(u[i].z, w[j].z, acc[i][j]); acc[i][j] = fmaf(u[i].w, w[j].w, acc[i][j]);
+      }
+  }
+}
+// acc[i][j] += sum_m U[ty + 16 i][m] V[m][4 tx + j]
+__device__ __forceinline__ void tile_mul_nn(float (&acc)[4][4], const float (*U)[CS], const float (*V)[CS]) {
+  const int ty = threadIdx.x >> 4, tx = threadIdx.x & 15;
+#pragma unroll 4
+  for (int m = 0; m < CB; m += 4) {
+    float4 u[4], w[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      u[i] = *reinterpret_cast<const float4*>(&U[ty + 16 * i][m]);
+      w[i] = *reinterpret_cast<const float4*>(&V[m + i][4 * tx]);
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const float ui[4] = {u[i].x, u[i].y, u[i].z, u[i].w};
+#pragma unroll
+      for (int m2 = 0; m2 < 4; ++m2) {
+        acc[i][0] = fmaf(ui[m2], w[m2].x, acc[i][0]); acc[i][1] = fmaf(ui[m2], w[m2].y, acc[i][1]);
+        acc[i][2] = fmaf(ui[m2], w[m2].z, acc[i][2]); acc[i][3] = fmaf(ui[m2], w[m2].w, acc[i][3]);
+      }
+    }
+  }
+}
+
+// One 64 x 64 tile of panel step kb per CTA.  Blocks [ob, kb) are the earlier panels of the same outer block,
+// whose updates have not been applied to this tile yet:
+//   row block i > kb:     A[i, kb] <- (A[i, kb] - sum_p A[i, p] A[kb, p]^T) inv^T
+//   column block c < kb:  X[kb, c] <- -inv (S[kb, c] + sum_p A[kb, p] X[p, c])
+// The sums run before the wait for the diagonal kernel.  The CTA of a row block inside the outer block
+// (i < obe) then brings its diagonal block up to date with the tile it holds, A[i, i] -= A[i, kb] A[i, kb]^T,
+// so that the next diagonal kernel finds a finished block.
 __global__ void __launch_bounds__(256)
-chol_tiles_kernel(float* __restrict__ A, float* __restrict__ X, int K, int kb, int tiles_below) {
-  __shared__ float a[CB][CPAD];
-  __shared__ float inv[CB][CPAD];
+chol_tiles_kernel(float* __restrict__ A, float* __restrict__ X, int K, int kb, int ob, int obe, int tiles_below, int vec) {
+  __shared__ __align__(16) float U[CB][CS];
+  __shared__ __align__(16) float V[CB][CS];
   const int r0 = kb * CB;
   const int nb = min(CB, K - r0);
-  const int tid = threadIdx.x;
+  const int tid = threadIdx.x, ty = tid >> 4, tx = tid & 15;
   const int bid = blockIdx.x;
-  const int tr = (tid >> 4) * 4, tc = (tid & 15) * 4;
   const bool below = bid < tiles_below;
-  const int p0 = (kb + 1) * CB + bid * CB;                 // (2): first row of the panel tile
-  const int c0 = (bid - tiles_below) * CB;                 // (4): first column of the row-block tile
-  for (int idx = tid; idx < CB * CB; idx += 256) {
-    const int i = idx / CB, j = idx % CB;
-    if (below) a[i][j] = (p0 + i < K && j < nb) ? A[(int64_t)(p0 + i) * K + r0 + j] : 0.f;
-    else       a[i][j] = (i < nb) ? X[(int64_t)(r0 + i) * K + c0 + j] : 0.f;
-  }
-  asm volatile("griddepcontrol.wait;" ::: "memory");
-  for (int idx = tid; idx < CB * CB; idx += 256) {
-    const int i = idx / CB, j = idx % CB;
-    inv[i][j] = (i < nb && j <= i) ? X[(int64_t)(r0 + i) * K + r0 + j] : 0.f;
+  const int ib = kb + 1 + bid;                             // row block of a tile below
+  const int i0 = ib * CB;
+  const int c0 = (bid - tiles_below) * CB;                 // first column of a tile of the inverse
+  float4 fu[4], fv[4];
+  float own[4][4], acc[4][4];
+  const int p_first = below ? ob : max(ob, bid - tiles_below);
+  auto fetch_pair = [&](int p) {
+    tile_fetch(fu, A, K, below ? i0 : r0, p * CB, K, K, vec);
+    if (below) tile_fetch(fv, A, K, r0, p * CB, K, K, vec);
+    else       tile_fetch(fv, X, K, p * CB, c0, K, K, vec);
+  };
+  // the tile itself is complete but for the outer block's earlier panels
+  if (below) tile_fetch(fu, A, K, i0, r0, K, r0 + nb, vec);
+  else       tile_fetch(fu, X, K, r0, c0, r0 + nb, K, vec);
+  tile_put(U, fu);
+  if (p_first < kb) fetch_pair(p_first);
+  __syncthreads();
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) own[i][j] = below ? U[ty + 16 * i][tx + 16 * j] : U[ty + 16 * i][4 * tx + j];
+  for (int p = p_first; p < kb; ++p) {
+    __syncthreads();
+    tile_put(U, fu);
+    tile_put(V, fv);
+    __syncthreads();
+    if (p + 1 < kb) fetch_pair(p + 1);
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) acc[i][j] = 0.f;
+    if (below) tile_mul_nt(acc, U, V);
+    else       tile_mul_nn(acc, U, V);
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) own[i][j] = below ? own[i][j] - acc[i][j] : own[i][j] + acc[i][j];
   }
   __syncthreads();
-  float acc[4][4] = {};
-  if (below) {
-    // (2) panel tile below the diagonal block:  tile <- tile * inv^T
-    for (int m = 0; m < nb; ++m) {
-      float pv[4], qv[4];
 #pragma unroll
-      for (int i = 0; i < 4; ++i) { pv[i] = a[tr + i][m]; qv[i] = inv[tc + i][m]; }
+  for (int i = 0; i < 4; ++i)
 #pragma unroll
-      for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(pv[i], qv[j], acc[i][j]);
+    for (int j = 0; j < 4; ++j) {
+      if (below) U[ty + 16 * i][tx + 16 * j] = own[i][j];
+      else       U[ty + 16 * i][4 * tx + j] = own[i][j];
+      acc[i][j] = 0.f;
     }
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  tile_fetch(fv, X, K, r0, r0, r0 + nb, r0 + nb, vec);
+  tile_put(V, fv);
+  __syncthreads();
+  if (!below) {
+    tile_mul_nn(acc, V, U);
 #pragma unroll
     for (int i = 0; i < 4; ++i)
+      if (ty + 16 * i < nb) {
+        float* dst = X + (int64_t)(r0 + ty + 16 * i) * K + c0 + 4 * tx;
+        if (vec) *reinterpret_cast<float4*>(dst) = make_float4(-acc[i][0], -acc[i][1], -acc[i][2], -acc[i][3]);
+        else
 #pragma unroll
-      for (int j = 0; j < 4; ++j)
-        if (p0 + tr + i < K && tc + j < nb) A[(int64_t)(p0 + tr + i) * K + r0 + tc + j] = acc[i][j];
-  } else {
-    // (4) row block kb of the inverse:  X[kb, jt] <- -inv * S[kb, jt]
-    for (int m = 0; m < nb; ++m) {
-      float pv[4], qv[4];
-#pragma unroll
-      for (int i = 0; i < 4; ++i) { pv[i] = inv[tr + i][m]; qv[i] = a[m][tc + i]; }
-#pragma unroll
-      for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(pv[i], qv[j], acc[i][j]);
-    }
-#pragma unroll
-    for (int i = 0; i < 4; ++i)
-#pragma unroll
-      for (int j = 0; j < 4; ++j)
-        if (tr + i < nb) X[(int64_t)(r0 + tr + i) * K + c0 + tc + j] = -acc[i][j];
+          for (int j = 0; j < 4; ++j) dst[j] = -acc[i][j];
+      }
+    return;
   }
+  tile_mul_nt(acc, U, V);
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+      if (i0 + ty + 16 * i < K && tx + 16 * j < nb) A[(int64_t)(i0 + ty + 16 * i) * K + r0 + tx + 16 * j] = acc[i][j];
+  if (ib >= obe) return;
+  __syncthreads();
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) { U[ty + 16 * i][tx + 16 * j] = acc[i][j]; acc[i][j] = 0.f; }
+  __syncthreads();
+  tile_mul_nt(acc, U, U);
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+      if (i0 + ty + 16 * i < K && i0 + tx + 16 * j < K) A[(int64_t)(i0 + ty + 16 * i) * K + i0 + tx + 16 * j] -= acc[i][j];
 }
 
 // ---- final: L[i][j] = X[K-1-j][K-1-i] (i >= j), 0 above the diagonal -----------
@@ -376,9 +557,10 @@ extern "C" int jgq_damp_invert(float* W, int64_t N, float* H, int64_t K, float d
   if (cudaMemsetAsync(X, 0, (size_t)K * K * sizeof(float), s) != cudaSuccess)
     return fail(JGQ_ERR_CUDA, "damp_invert: memset failed");
 
-  // Two-level blocking: inside an outer block of COB panels the rank-64 updates only touch the
-  // block's own columns of A and its own rows of S; everything beyond the block gets one update of
-  // depth 64 * COB when the block is finished, which is where nearly all the arithmetic is.
+  // Two-level blocking: inside an outer block of COB panels the tile kernel applies the block's earlier
+  // panels itself; everything beyond the block gets one update of depth 64 * COB when the block is
+  // finished, which is where nearly all the arithmetic is.
+  const int vec = (Ki % 4 == 0) && aligned(A, 16) && aligned(X, 16);
   const int nblk = (int)cdiv(K, CB);
   for (int ob = 0; ob < nblk; ob += COB) {
     const int c_begin = ob * CB;                                   // first column of the outer block
@@ -386,35 +568,27 @@ extern "C" int jgq_damp_invert(float* W, int64_t N, float* H, int64_t K, float d
     for (int kb = ob; kb < std::min(nblk, ob + COB); ++kb) {
       const int r1 = std::min(Ki, (kb + 1) * CB);      // first row below the diagonal block
       const int below = Ki - r1;
-      const int nb = std::min(CB, Ki - kb * CB);
       const int tiles_below = below > 0 ? (int)cdiv(below, CB) : 0;
-      chol_diag_kernel<<<1, 256, 0, s>>>(A, X, Ki, kb, dev_status);
-      JGQ_LAUNCHED();
-      if (tiles_below + kb > 0) {
-        cudaLaunchConfig_t cfg;
-        memset(&cfg, 0, sizeof(cfg));
+      // both launches of a step may be placed while their predecessor is finishing; they wait inside
+      cudaLaunchAttribute attr[1];
+      attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+      attr[0].val.programmaticStreamSerializationAllowed = 1;
+      cudaLaunchConfig_t cfg;
+      memset(&cfg, 0, sizeof(cfg));
+      cfg.gridDim = dim3(1);
+      cfg.blockDim = dim3(256);
+      cfg.stream = s;
+      cfg.attrs = attr;
+      cfg.numAttrs = kb > 0 ? 1 : 0;       // the first one follows a memset, which signals nothing early
+      cudaError_t e = cudaLaunchKernelEx(&cfg, chol_diag_kernel, (const float*)A, X, Ki, kb, vec, dev_status);
+      note_launches(1);
+      if (e == cudaSuccess && tiles_below + kb > 0) {
         cfg.gridDim = dim3((unsigned)(tiles_below + kb));
-        cfg.blockDim = dim3(256);
-        cfg.stream = s;
-        cudaLaunchAttribute attr[1];
-        attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-        attr[0].val.programmaticStreamSerializationAllowed = 1;
-        cfg.attrs = attr;
         cfg.numAttrs = 1;
-        const cudaError_t e = cudaLaunchKernelEx(&cfg, chol_tiles_kernel, A, X, Ki, kb, tiles_below);
+        e = cudaLaunchKernelEx(&cfg, chol_tiles_kernel, A, X, Ki, kb, ob, std::min(nblk, ob + COB), tiles_below, vec);
         note_launches(1);
-        if (e != cudaSuccess) { cudaGetLastError(); return fail(JGQ_ERR_CUDA, "damp_invert: %s", cudaGetErrorString(e)); }
       }
-      if (c_end > r1) {
-        // (3) A[r1:, r1:c_end] -= P P[r1:c_end]^T (lower tiles) and (5) S[r1:c_end, :r1] += P[r1:c_end] X[k, :r1]
-        const float* P = A + (int64_t)r1 * K + (int64_t)kb * CB;
-        GemmParams g0 = make_gemm_params(P, K, P, K, A + (int64_t)r1 * K + r1, K, below, c_end - r1, nb,
-                                         -1.f, 1.f, 1);
-        GemmParams g1 = make_gemm_params(P, K, X + (int64_t)kb * CB * K, K, X + (int64_t)r1 * K, K,
-                                         c_end - r1, r1, nb, 1.f, 1.f, 0);
-        const int rc = launch_sgemm_dual(g0, true, g1, false, s);
-        if (rc) return rc;
-      }
+      if (e != cudaSuccess) { cudaGetLastError(); return fail(JGQ_ERR_CUDA, "damp_invert: %s", cudaGetErrorString(e)); }
     }
     if (c_end < Ki) {
       // the block's whole panel Pb = A[c_end:, c_begin:c_end] at once:
