@@ -105,6 +105,12 @@ int jgq_col_params(const float* W, int64_t K, int64_t N, int maxq,
 size_t jgq_hessian_workspace_bytes(int64_t n, int64_t K, int x_dtype);
 int jgq_hessian_accum(const void* X, int x_dtype, int64_t n, int64_t K, float* H,
                       void* ws, size_t ws_bytes, int32_t* dev_status, void* stream);
+/* Several batches in one call: X is a HOST array of `count` device pointers, n their row counts (all > 0).  The result is
+ * bit for bit that of jgq_hessian_accum called for one batch after the other; from K = 512 up to 16 batches share one
+ * launch. */
+size_t jgq_hessian_batches_workspace_bytes(const int64_t* n, int count, int64_t K, int x_dtype);
+int jgq_hessian_accum_batches(const void* const* X, const int64_t* n, int count, int x_dtype, int64_t K, float* H,
+                              void* ws, size_t ws_bytes, int32_t* dev_status, void* stream);
 int jgq_hessian_finalize(float* H, int64_t K, double n_total, void* stream);
 
 /* Token-sharded accumulation over several GPUs (no counterpart in the reference, which pins one GPU,

@@ -33,6 +33,8 @@ SIGNATURES = {
     'jgq_col_params': (_int, [_vp, _i64, _i64, _int, _vp, _vp, _vp]),
     'jgq_hessian_workspace_bytes': (_sz, [_i64, _i64, _int]),
     'jgq_hessian_accum': (_int, [_vp, _int, _i64, _i64, _vp, _vp, _sz, _vp, _vp]),
+    'jgq_hessian_batches_workspace_bytes': (_sz, [_vp, _int, _i64, _int]),
+    'jgq_hessian_accum_batches': (_int, [_vp, _vp, _int, _int, _i64, _vp, _vp, _sz, _vp, _vp]),
     'jgq_hessian_finalize': (_int, [_vp, _i64, C.c_double, _vp]),
     'jgq_hessian_lower_elems': (_sz, [_i64]),
     'jgq_hessian_pack_lower': (_int, [_vp, _i64, _vp, _vp]),

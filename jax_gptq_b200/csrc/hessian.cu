@@ -21,17 +21,48 @@ __global__ void to_f32_kernel(const T* __restrict__ in, float* __restrict__ out,
     out[t] = to_f32<T>(in[t]);
 }
 
-// H[i][j] += sum_z part[z][i][j] for tiles on or below the diagonal
-__global__ void reduce_splits_kernel(float* __restrict__ H, const float* __restrict__ part,
-                                     int K, int splits) {
-  const int j = blockIdx.x * blockDim.x + threadIdx.x;
+// H[i][j] += sum over the slices z of part[z][i][j], batch after batch, for tiles on or below the diagonal.
+// Bound by HBM / L2: `kVec` (K % 4 == 0) moves 16 bytes per lane, four slices' loads in flight.
+struct ReduceParams { int count; int start[HESS_MAX_BATCHES + 1]; };
+template <int V>
+__global__ void reduce_splits_kernel(float* __restrict__ H, const float* __restrict__ part, int K, const ReduceParams rp) {
+  const int j = V * (blockIdx.x * blockDim.x + threadIdx.x);
   const int i = blockIdx.y * blockDim.y + threadIdx.y;
   if (i >= K || j >= K) return;
   if ((j / GBN) > (i / GBM)) return;
-  const int64_t o = (int64_t)i * K + j;
-  float s = 0.f;
-  for (int z = 0; z < splits; ++z) s += part[(int64_t)z * K * K + o];
-  H[o] += s;
+  const int64_t o = (int64_t)i * K + j, stride = (int64_t)K * K;
+  float h[V];
+#pragma unroll
+  for (int v = 0; v < V; ++v) h[v] = H[o + v];
+  for (int b = 0; b < rp.count; ++b) {
+    float s[V];
+#pragma unroll
+    for (int v = 0; v < V; ++v) s[v] = 0.f;
+    const int z1 = rp.start[b + 1];
+#pragma unroll 4
+    for (int z = rp.start[b]; z < z1; ++z) {
+      if (V == 4) {
+        const float4 q = __ldcs(reinterpret_cast<const float4*>(part + z * stride + o));
+        s[0] += q.x; s[1 % V] += q.y; s[2 % V] += q.z; s[3 % V] += q.w;
+      } else {
+        s[0] += part[z * stride + o];
+      }
+    }
+#pragma unroll
+    for (int v = 0; v < V; ++v) h[v] += s[v];
+  }
+#pragma unroll
+  for (int v = 0; v < V; ++v) H[o + v] = h[v];
+}
+
+static int reduce_splits(float* H, const float* part, int64_t K, const ReduceParams& rp, cudaStream_t s) {
+  const bool vec = K % 4 == 0 && aligned(H, 16) && aligned(part, 16);
+  dim3 blk(32, 8), grd((unsigned)cdiv(K, vec ? 128 : 32), (unsigned)cdiv(K, 8));
+  prefer_shared_carveout<reduce_splits_kernel<1>>();
+  prefer_shared_carveout<reduce_splits_kernel<4>>();
+  if (vec) reduce_splits_kernel<4><<<grd, blk, 0, s>>>(H, part, (int)K, rp);
+  else     reduce_splits_kernel<1><<<grd, blk, 0, s>>>(H, part, (int)K, rp);
+  return check_launch("hessian_reduce");
 }
 
 // lower triangle / n  ->  both triangles
@@ -134,11 +165,9 @@ extern "C" int jgq_hessian_accum(const void* X, int x_dtype, int64_t n, int64_t 
     int rc = launch_hessian_umma(pl, X, x_dtype, n, K, H, ws, dev_status, s);
     if (rc) return rc;
     if (pl.S > 1) {
-      const float* part = (const float*)((const char*)ws + 2 * pl.plane_bytes);
-      dim3 blk(32, 8), grd((unsigned)cdiv(K, 32), (unsigned)cdiv(K, 8));
-      prefer_shared_carveout<reduce_splits_kernel>();
-      reduce_splits_kernel<<<grd, blk, 0, s>>>(H, part, (int)K, pl.S);
-      return check_launch("hessian_reduce");
+      ReduceParams rp;
+      rp.count = 1; rp.start[0] = 0; rp.start[1] = pl.S;
+      return reduce_splits(H, (const float*)((const char*)ws + 2 * pl.plane_bytes), K, rp, s);
     }
     return JGQ_OK;
   }
@@ -160,9 +189,55 @@ extern "C" int jgq_hessian_accum(const void* X, int x_dtype, int64_t n, int64_t 
   int rc = launch_sgemm(false, false, Xf, K, Xf, K, part, K, (int)K, (int)K, (int)n, 1.f, 0.f, 1, s,
                         splits, (int64_t)K * K);
   if (rc) return rc;
-  dim3 blk(32, 8), grd((unsigned)cdiv(K, 32), (unsigned)cdiv(K, 8));
-  reduce_splits_kernel<<<grd, blk, 0, s>>>(H, part, (int)K, splits);
-  return check_launch("hessian_accum");
+  ReduceParams rp;
+  rp.count = 1; rp.start[0] = 0; rp.start[1] = splits;
+  return reduce_splits(H, part, K, rp, s);
+}
+
+extern "C" size_t jgq_hessian_batches_workspace_bytes(const int64_t* n, int count, int64_t K, int x_dtype) {
+  if (!n || count <= 0 || K <= 0) return 0;
+  const HessBatchesPlan bp = plan_hessian_batches(n, count, K, x_dtype);
+  if (bp.use) return 2 * bp.plane_bytes + bp.part_bytes;
+  if (count >= 4)                                     // too many for one launch (or for its buffers): two halves
+    return std::max(jgq_hessian_batches_workspace_bytes(n, count / 2, K, x_dtype),
+                    jgq_hessian_batches_workspace_bytes(n + count / 2, count - count / 2, K, x_dtype));
+  size_t need = 0;
+  for (int b = 0; b < count; ++b) need = std::max(need, jgq_hessian_workspace_bytes(n[b], K, x_dtype));
+  return need;
+}
+
+extern "C" int jgq_hessian_accum_batches(const void* const* X, const int64_t* n, int count, int x_dtype, int64_t K, float* H,
+                                         void* ws, size_t ws_bytes, int32_t* dev_status, void* stream) {
+  JGQ_REQUIRE(X && n && count > 0, JGQ_ERR_ARG, "hessian_accum_batches: no batches");
+  JGQ_REQUIRE(x_dtype == JGQ_F32 || x_dtype == JGQ_F16 || x_dtype == JGQ_BF16, JGQ_ERR_ARG,
+              "hessian_accum_batches: X dtype must be f32/f16/bf16");
+  JGQ_REQUIRE(K > 0 && K <= 46340 && H, JGQ_ERR_ARG, "hessian_accum_batches: bad K=%lld or null H", (long long)K);
+  for (int b = 0; b < count; ++b)
+    JGQ_REQUIRE(X[b] && n[b] > 0 && n[b] <= 2147483647LL, JGQ_ERR_ARG, "hessian_accum_batches: batch %d is null or has %lld rows", b, (long long)n[b]);
+  const size_t need = jgq_hessian_batches_workspace_bytes(n, count, K, x_dtype);
+  JGQ_REQUIRE(ws_bytes >= need && (need == 0 || ws), JGQ_ERR_WORKSPACE,
+              "hessian_accum_batches: workspace %zu < %zu bytes", ws_bytes, need);
+  JGQ_REQUIRE(need == 0 || aligned(ws, 256), JGQ_ERR_ALIGN, "hessian_accum_batches: workspace must be 256-byte aligned");
+  const HessBatchesPlan bp = plan_hessian_batches(n, count, K, x_dtype);
+  if (!bp.use && count >= 4) {
+    const int h = count / 2;
+    const int rc = jgq_hessian_accum_batches(X, n, h, x_dtype, K, H, ws, ws_bytes, dev_status, stream);
+    return rc ? rc : jgq_hessian_accum_batches(X + h, n + h, count - h, x_dtype, K, H, ws, ws_bytes, dev_status, stream);
+  }
+  if (!bp.use) {
+    for (int b = 0; b < count; ++b) {
+      const int rc = jgq_hessian_accum(X[b], x_dtype, n[b], K, H, ws, ws_bytes, dev_status, stream);
+      if (rc) return rc;
+    }
+    return JGQ_OK;
+  }
+  for (int b = 0; b < count; ++b)
+    JGQ_REQUIRE(aligned(X[b], 16) && aligned(H, 16), JGQ_ERR_ALIGN, "hessian_accum_batches: X and H must be 16-byte aligned");
+  ReduceParams rp;
+  rp.count = count;
+  const int rc = launch_hessian_batches(bp, X, n, count, x_dtype, K, H, ws, dev_status, rp.start, (cudaStream_t)stream);
+  if (rc || bp.mode == 1) return rc;
+  return reduce_splits(H, (const float*)((const char*)ws + 2 * bp.plane_bytes), K, rp, (cudaStream_t)stream);
 }
 
 extern "C" size_t jgq_hessian_lower_elems(int64_t K) {

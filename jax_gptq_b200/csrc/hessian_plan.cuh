@@ -10,4 +10,11 @@ HessPlan plan_hessian_umma(int64_t n, int64_t K, int x_dtype);
 int launch_hessian_umma(const HessPlan& pl, const void* X, int x_dtype, int64_t n, int64_t K, float* H, void* ws,
                         int32_t* status, cudaStream_t s);
 
+// several batches in one launch of the CTA-pair kernel (mode: see plan_hessian_batches)
+constexpr int HESS_MAX_BATCHES = 16, HESS_MAX_SEGS = 128;
+struct HessBatchesPlan { int use; int mode; int nseg; int parts; size_t plane_bytes; size_t part_bytes; HessPlan batch[HESS_MAX_BATCHES]; };
+HessBatchesPlan plan_hessian_batches(const int64_t* n, int count, int64_t K, int x_dtype);
+int launch_hessian_batches(const HessBatchesPlan& bp, const void* const* X, const int64_t* n, int count, int x_dtype,
+                           int64_t K, float* H, void* ws, int32_t* status, int* part_start, cudaStream_t s);
+
 }  // namespace jgq

@@ -72,12 +72,29 @@ struct HessParams {
   int withhold_first_chain;   // test hook: the MMA warp never signals its first finished chain (see launch_hessian_umma)
 };
 
-template <typename T>
-__global__ void split_bf16_kernel(const T* __restrict__ X, __nv_bfloat16* __restrict__ P0,
-                                  __nv_bfloat16* __restrict__ P1, int64_t total4) {
+// Work table of the CTA-pair kernel.  A run is what one pair does for its tile: a list of segments (token ranges of
+// one batch) it sums one after the other.  A segment's sum is stored to a slice buffer, added to one, or added to H.
+struct HessSeg { int map, tok0, tok_end, part, add; };        // part < 0: H
+struct HessPairParams {
+  CUtensorMap maps[2 * HESS_MAX_BATCHES];                     // batch b: planes 2 b and 2 b + 1
+  HessSeg seg[HESS_MAX_SEGS];
+  int run_start[HESS_MAX_SEGS + 1];
+  int K, planes, fmt, nseg;
+  float* H; float* parts; int64_t part_stride;
+  int32_t* status;
+  int withhold_first_chain;
+};
+
+// fp32 batches -> two bf16 planes each, one batch per blockIdx.y
+struct SplitParams { const float* X[HESS_MAX_BATCHES]; __nv_bfloat16* P0[HESS_MAX_BATCHES]; __nv_bfloat16* P1[HESS_MAX_BATCHES]; int64_t total4[HESS_MAX_BATCHES]; };
+__global__ void split_bf16_kernel(const __grid_constant__ SplitParams p) {
+  const float4* X = reinterpret_cast<const float4*>(p.X[blockIdx.y]);
+  uint2* P0 = reinterpret_cast<uint2*>(p.P0[blockIdx.y]);
+  uint2* P1 = reinterpret_cast<uint2*>(p.P1[blockIdx.y]);
+  const int64_t total4 = p.total4[blockIdx.y];
   for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < total4;
        t += (int64_t)gridDim.x * blockDim.x) {
-    const float4 v = reinterpret_cast<const float4*>(X)[t];
+    const float4 v = X[t];
     const float x[4] = {v.x, v.y, v.z, v.w};
     __nv_bfloat16 hi[4], lo[4];
 #pragma unroll
@@ -90,8 +107,8 @@ __global__ void split_bf16_kernel(const T* __restrict__ X, __nv_bfloat16* __rest
     h.y = (uint32_t)__bfloat16_as_ushort(hi[2]) | ((uint32_t)__bfloat16_as_ushort(hi[3]) << 16);
     l.x = (uint32_t)__bfloat16_as_ushort(lo[0]) | ((uint32_t)__bfloat16_as_ushort(lo[1]) << 16);
     l.y = (uint32_t)__bfloat16_as_ushort(lo[2]) | ((uint32_t)__bfloat16_as_ushort(lo[3]) << 16);
-    reinterpret_cast<uint2*>(P0)[t] = h;
-    reinterpret_cast<uint2*>(P1)[t] = l;
+    P0[t] = h;
+    P1[t] = l;
   }
 }
 
@@ -361,8 +378,7 @@ __device__ __forceinline__ void mma_commit_pair(uint32_t bar_cluster_addr) {
 }
 
 __global__ void __launch_bounds__(HT_THREADS, 1)
-hessian_pair_kernel(const __grid_constant__ CUtensorMap map0, const __grid_constant__ CUtensorMap map1,
-                    const HessParams p) {
+hessian_pair_kernel(const __grid_constant__ HessPairParams p) {
   using namespace umma;
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   uint8_t* smem = smem_raw;
@@ -377,8 +393,8 @@ hessian_pair_kernel(const __grid_constant__ CUtensorMap map0, const __grid_const
   const uint32_t rank = cluster_ctarank();           // 0: issues the pair's MMAs
   const int pair = blockIdx.x >> 1;
 
-  // ---- which 256 x 256 tile / token slice ----
-  const int slice = pair / p.nseg;
+  // ---- which 256 x 256 tile / run of segments ----
+  const int run = pair / p.nseg;
   int seg = pair % p.nseg;
   int I = 0;
   while (seg > I) { seg -= I + 1; ++I; }             // row panel I has tiles 0..I
@@ -386,10 +402,7 @@ hessian_pair_kernel(const __grid_constant__ CUtensorMap map0, const __grid_const
   const int row0 = I * 256 + 128 * (int)rank;        // this CTA's 128 rows
   const int col0 = seg * 256;
   const int colh = col0 + 128 * (int)rank;           // its half of the B operand
-  const int tok0 = slice * p.tokens_per_slice;
-  const int tok_end = min(p.n, tok0 + p.tokens_per_slice);
-  const int nstages = (tok_end - tok0 + HT_BK - 1) / HT_BK;
-  const int nchains = (nstages + HT_CHUNK - 1) / HT_CHUNK;
+  const int s_begin = p.run_start[run], s_end = p.run_start[run + 1];
 
   const bool misaligned = (smem_u32(smem) & 1023u) != 0u;
   if (threadIdx.x == 0) {
@@ -398,8 +411,8 @@ hessian_pair_kernel(const __grid_constant__ CUtensorMap map0, const __grid_const
     *abort_flag = misaligned ? 1 : 0;
     if (misaligned && p.status) atomicOr(p.status, JGQ_STATUS_LAYOUT);
     fence_barrier_init();
-    prefetch_tensormap(&map0);
-    if (p.planes > 1) prefetch_tensormap(&map1);
+    prefetch_tensormap(&p.maps[2 * p.seg[s_begin].map]);
+    if (p.planes > 1) prefetch_tensormap(&p.maps[2 * p.seg[s_begin].map + 1]);
   }
   if (warp == 1) {
     asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"((uint32_t)HT_TMEM_COLS) : "memory");
@@ -423,23 +436,28 @@ hessian_pair_kernel(const __grid_constant__ CUtensorMap map0, const __grid_const
     int st = 0;
     uint32_t ph = 0;
     int issued = 0;
-    for (int kc = 0; kc < nstages; ++kc) {
-      if (kc >= HP_STAGES && !__all_sync(0xffffffffu, mbar_wait(&empty_bar[st], ph ^ 1, abort_flag))) break;
-      if (lane == 0) {
-        if (rank == 0) mbar_expect_tx(&full_bar[st], 2 * stage_tx);       // the bytes of both CTAs
-        const int tok = tok0 + kc * HT_BK;
-        uint8_t* sb = smem + st * HP_STAGE_BYTES;
-        const uint32_t bar = full0 + (uint32_t)(st * 8);
-        for (int pl = 0; pl < p.planes; ++pl) {
-          const CUtensorMap* m = pl == 0 ? &map0 : &map1;
-          uint8_t* pb = sb + pl * HP_PLANE_BYTES;
-          for (int g = 0; g < 2; ++g) tma_load_2d_pair(pb + g * HT_BOX_BYTES, m, row0 + 64 * g, tok, bar);
-          for (int g = 0; g < boxes_b; ++g) tma_load_2d_pair(pb + (2 + g) * HT_BOX_BYTES, m, colh + 64 * g, tok, bar);
+    bool ok = true;
+    for (int sg = s_begin; sg < s_end && ok; ++sg) {
+      const HessSeg& g = p.seg[sg];
+      const CUtensorMap* m0 = &p.maps[2 * g.map];
+      for (int tok = g.tok0; tok < g.tok_end && ok; tok += HT_BK) {
+        if (issued >= HP_STAGES) ok = __all_sync(0xffffffffu, mbar_wait(&empty_bar[st], ph ^ 1, abort_flag));
+        if (!ok) break;
+        if (lane == 0) {
+          if (rank == 0) mbar_expect_tx(&full_bar[st], 2 * stage_tx);       // the bytes of both CTAs
+          uint8_t* sb = smem + st * HP_STAGE_BYTES;
+          const uint32_t bar = full0 + (uint32_t)(st * 8);
+          for (int pl = 0; pl < p.planes; ++pl) {
+            const CUtensorMap* m = m0 + pl;
+            uint8_t* pb = sb + pl * HP_PLANE_BYTES;
+            for (int q = 0; q < 2; ++q) tma_load_2d_pair(pb + q * HT_BOX_BYTES, m, row0 + 64 * q, tok, bar);
+            for (int q = 0; q < boxes_b; ++q) tma_load_2d_pair(pb + (2 + q) * HT_BOX_BYTES, m, colh + 64 * q, tok, bar);
+          }
         }
+        __syncwarp();
+        ++issued;
+        if (++st == HP_STAGES) { st = 0; ph ^= 1; }
       }
-      __syncwarp();
-      issued = kc + 1;
-      if (++st == HP_STAGES) { st = 0; ph ^= 1; }
     }
     if (*abort_flag && issued > 0) {
       // after a timed-out wait boxes may still be in flight: give them a bounded time to land
@@ -461,8 +479,10 @@ hessian_pair_kernel(const __grid_constant__ CUtensorMap map0, const __grid_const
       uint32_t sb16 = smem0 >> 4;
       const uint32_t stage16 = (uint32_t)HP_STAGE_BYTES >> 4;
       const uint32_t my_empty = smem_u32(&empty_bar[0]), my_accf = smem_u32(&accf_bar[0]);
-      int kc = 0;
-      for (int c = 0; c < nchains && ok; ++c) {
+      int c = 0;                                      // chains of all segments, counted through
+      for (int sg = s_begin; sg < s_end && ok; ++sg) {
+      const int nstages = (p.seg[sg].tok_end - p.seg[sg].tok0 + HT_BK - 1) / HT_BK;
+      for (int kc = 0; kc < nstages && ok; ++c) {
         const int b = c & 1;
         if (c >= 2) {
           ok = __all_sync(0xffffffffu, mbar_wait(&acce_bar[b], ((uint32_t)(c >> 1) & 1u) ^ 1u, abort_flag));
@@ -503,6 +523,7 @@ hessian_pair_kernel(const __grid_constant__ CUtensorMap map0, const __grid_const
         }
         __syncwarp();
       }
+      }
     }
   } else {
     // ===================== long accumulation + epilogue (both CTAs) =====================
@@ -510,37 +531,41 @@ hessian_pair_kernel(const __grid_constant__ CUtensorMap map0, const __grid_const
     const int q = warp & 3;
     const int half = e >> 2;
     const int cbeg = half * (HT_N / 2);
+    const int i = row0 + 32 * q + lane;
     float acc[HT_N / 2];
 #pragma unroll
-    for (int i = 0; i < HT_N / 2; ++i) acc[i] = 0.f;
+    for (int v = 0; v < HT_N / 2; ++v) acc[v] = 0.f;
     bool ok = true;
-    for (int c = 0; c < nchains && ok; ++c) {
-      const int b = c & 1;
-      ok = __all_sync(0xffffffffu, mbar_wait(&accf_bar[b], (uint32_t)(c >> 1) & 1u, abort_flag));
-      if (!ok) break;
-      tc_fence_after();
+    int c = 0;
+    for (int sg = s_begin; sg < s_end && ok; ++sg) {
+      const HessSeg& g = p.seg[sg];
+      const int nchains = (g.tok_end - g.tok0 + HT_BK * HT_CHUNK - 1) / (HT_BK * HT_CHUNK);
+      for (const int c_end = c + nchains; c < c_end && ok; ++c) {
+        const int b = c & 1;
+        ok = __all_sync(0xffffffffu, mbar_wait(&accf_bar[b], (uint32_t)(c >> 1) & 1u, abort_flag));
+        if (!ok) break;
+        tc_fence_after();
 #pragma unroll
-      for (int cc = 0; cc < HT_N / 2; cc += 32) {
-        uint32_t r[32];
-        tmem_ld_32x32(tmem_acc + (uint32_t)(b * HT_N) + ((uint32_t)(32 * q) << 16) + (uint32_t)(cbeg + cc), r);
-        tmem_ld_wait();
+        for (int cc = 0; cc < HT_N / 2; cc += 32) {
+          uint32_t r[32];
+          tmem_ld_32x32(tmem_acc + (uint32_t)(b * HT_N) + ((uint32_t)(32 * q) << 16) + (uint32_t)(cbeg + cc), r);
+          tmem_ld_wait();
 #pragma unroll
-        for (int v = 0; v < 32; ++v) acc[cc + v] = __fadd_rn(acc[cc + v], __uint_as_float(r[v]));
+          for (int v = 0; v < 32; ++v) acc[cc + v] = __fadd_rn(acc[cc + v], __uint_as_float(r[v]));
+        }
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive_cluster(acce0 + (uint32_t)(b * 8));
       }
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive_cluster(acce0 + (uint32_t)(b * 8));
-    }
-    if (ok) {
-      float* out = p.out + (int64_t)slice * p.slice_stride;
-      const int i = row0 + 32 * q + lane;
+      if (!ok) break;
+      // the segment's sum goes out; the MMA warp is already two chains into the next one
       if (i < p.K) {
-        float* dst = out + (int64_t)i * p.K + col0 + cbeg;
+        float* dst = (g.part < 0 ? p.H : p.parts + (int64_t)g.part * p.part_stride) + (int64_t)i * p.K + col0 + cbeg;
 #pragma unroll
         for (int v = 0; v < HT_N / 8; ++v) {
           if (col0 + cbeg + 4 * v < p.K) {          // K % 8 == 0: the four columns are inside together
             float4 o = make_float4(acc[4 * v], acc[4 * v + 1], acc[4 * v + 2], acc[4 * v + 3]);
-            if (p.S == 1) {
+            if (g.add) {
               const float4 h = *reinterpret_cast<const float4*>(dst + 4 * v);
               o.x += h.x; o.y += h.y; o.z += h.z; o.w += h.w;
             }
@@ -548,6 +573,8 @@ hessian_pair_kernel(const __grid_constant__ CUtensorMap map0, const __grid_const
           }
         }
       }
+#pragma unroll
+      for (int v = 0; v < HT_N / 2; ++v) acc[v] = 0.f;
     }
   }
   }
@@ -612,6 +639,134 @@ HessPlan plan_hessian_umma(int64_t n, int64_t K, int x_dtype) {
   return pl;
 }
 
+static void split_planes(const SplitParams& sp, int count, int64_t max_total4, cudaStream_t s) {
+  const int blocks = (int)std::min<int64_t>(cdiv(max_total4, 256), std::max<int64_t>(1, (int64_t)sm_count() * 16 / count));
+  prefer_shared_carveout<split_bf16_kernel>();
+  split_bf16_kernel<<<dim3((unsigned)blocks, (unsigned)count), 256, 0, s>>>(sp);
+  JGQ_LAUNCHED();
+}
+
+static int launch_pair(HessPairParams& p, int runs, cudaStream_t s) {
+  // Test hook for the bounded waits: with JGQ_TEST_WITHHOLD_COMMIT set (read at every launch) the MMA warp keeps its
+  // first "chain finished" signal to itself; the waits of every role then run out their budget, the kernel returns
+  // without writing H and reports JGQ_STATUS_TIMEOUT.  Nothing faults and nothing spins without a limit.
+  p.withhold_first_chain = getenv("JGQ_TEST_WITHHOLD_COMMIT") ? 1 : 0;
+  struct PairAttrTag {};
+  once_per_device<PairAttrTag>([]() {
+    cudaFuncSetAttribute(hessian_pair_kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 0);
+    cudaGetLastError();
+    return (int)cudaFuncSetAttribute(hessian_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     HP_RING_BYTES + HT_BAR_BYTES);
+  });
+  cudaLaunchConfig_t cfg;
+  memset(&cfg, 0, sizeof(cfg));
+  cfg.gridDim = dim3((unsigned)(2 * p.nseg * runs));
+  cfg.blockDim = dim3(HT_THREADS);
+  cfg.dynamicSmemBytes = HP_RING_BYTES + HT_BAR_BYTES;
+  cfg.stream = s;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = 2; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, hessian_pair_kernel, p);
+  note_launches(1);
+  if (e != cudaSuccess) { cudaGetLastError(); return fail(JGQ_ERR_CUDA, "hessian_pair: %s", cudaGetErrorString(e)); }
+  return JGQ_OK;
+}
+
+// How several batches share a launch of the pair kernel.  Every batch keeps the token slices it has alone, and H takes
+// the batches' sums in order, so the result is that of one call per batch.  What is free is who does what:
+//   per tile   a pair walks all batches of its tile and adds each sum to H (only when no batch is sliced): no buffers;
+//   per batch  a pair walks the slices of one batch, the batch's sum goes to a buffer;
+//   per slice  every slice has its pair and its buffer, as in a call per batch.
+// The estimate: waves over the pairs, a pair costing its tokens, about 350 more for its set-up and pipeline fill
+// (1000 with one plane, where a token is a third of the work) and 100 per further segment; the buffers' traffic at 34
+// tokens (100) per 6 MB.  Measured at K = 3072, sixteen fp32 batches of 4096: one call per batch 4.0 ms, two calls of eight per batch 2.9 ms (2.05 if they were one batch).
+HessBatchesPlan plan_hessian_batches(const int64_t* n, int count, int64_t K, int x_dtype) {
+  HessBatchesPlan bp;
+  memset(&bp, 0, sizeof(bp));
+  if (count < 2 || count > HESS_MAX_BATCHES) return bp;
+  int64_t total = 0, nmax = 0, tpsmax = 0;
+  int slices = 0, nseg = 0;
+  for (int b = 0; b < count; ++b) {
+    const HessPlan pl = plan_hessian_umma(n[b], K, x_dtype);
+    if (!pl.use || pl.panel != 256) return bp;
+    bp.batch[b] = pl;
+    total += n[b]; nmax = std::max(nmax, n[b]); tpsmax = std::max<int64_t>(tpsmax, pl.tokens_per_slice);
+    slices += pl.S; nseg = pl.nseg;
+    bp.plane_bytes += pl.plane_bytes;
+  }
+  if (slices > HESS_MAX_SEGS) return bp;
+  const int pairs = std::max(1, sm_count() / 2);
+  const bool two = x_dtype == JGQ_F32;
+  const double setup = two ? 350 : 1000, tok_per_byte = (two ? 34.0 : 100.0) / 6e6;
+  const double square = (double)K * K * sizeof(float);
+  auto waves = [&](int64_t units) { return (double)cdiv(units, pairs); };
+  const size_t cap = (size_t)512 << 20;
+  double best = 1e300;
+  auto offer = [&](int mode, double cost, size_t buffers) {
+    if (buffers * (size_t)square <= cap && cost < best) { best = cost; bp.mode = mode; bp.parts = (int)buffers; }
+  };
+  if (slices == count) offer(1, waves(nseg) * (total + setup + 100.0 * count), 0);
+  offer(2, waves((int64_t)nseg * count) * (nmax + setup + 100.0 * (double)slices / count) + 1.1 * square * count * tok_per_byte, count);
+  offer(3, waves((int64_t)nseg * slices) * (tpsmax + setup) + 1.1 * square * slices * tok_per_byte, slices);
+  bp.use = bp.mode != 0;
+  bp.nseg = nseg;
+  bp.part_bytes = align_up((size_t)bp.parts * K * K * sizeof(float), 256);
+  return bp;
+}
+
+// H (lower blocks) += the sums of the batches; the caller adds the slice buffers to H (hessian.cu).
+int launch_hessian_batches(const HessBatchesPlan& bp, const void* const* X, const int64_t* n, int count, int x_dtype,
+                           int64_t K, float* H, void* ws, int32_t* status, int* part_start, cudaStream_t s) {
+  HessPairParams p;
+  memset(&p, 0, sizeof(p));
+  uint8_t* w = (uint8_t*)ws;
+  SplitParams sp;
+  int64_t max4 = 0;
+  const void* plane[2 * HESS_MAX_BATCHES];
+  const bool two = x_dtype == JGQ_F32;
+  for (int b = 0; b < count; ++b) {
+    plane[2 * b] = plane[2 * b + 1] = X[b];
+    if (two) {
+      plane[2 * b] = w; plane[2 * b + 1] = w + bp.batch[b].plane_bytes;
+      w += 2 * bp.batch[b].plane_bytes;
+      sp.X[b] = (const float*)X[b]; sp.P0[b] = (__nv_bfloat16*)plane[2 * b]; sp.P1[b] = (__nv_bfloat16*)plane[2 * b + 1];
+      sp.total4[b] = n[b] * K / 4;
+      max4 = std::max(max4, sp.total4[b]);
+    }
+  }
+  if (two) split_planes(sp, count, max4, s);
+  for (int b = 0; b < count; ++b)
+    for (int pl = 0; pl < 2; ++pl) {
+      const int rc = encode_tmap_2d_b16(&p.maps[2 * b + pl], plane[2 * b + pl], (uint64_t)K, (uint64_t)n[b], (uint64_t)K * 2, 64, HT_BK);
+      if (rc) return rc;
+    }
+  p.K = (int)K; p.planes = two ? 2 : 1; p.fmt = x_dtype == JGQ_F16 ? 0 : 1; p.nseg = bp.nseg;
+  p.H = H; p.parts = (float*)w; p.part_stride = K * K; p.status = status;
+  int segs = 0, runs = 0, part = 0;
+  for (int b = 0; b < count; ++b) {
+    const HessPlan& pl = bp.batch[b];
+    if (part_start) part_start[b] = part;
+    if (bp.mode == 2 || (bp.mode == 1 && b == 0)) p.run_start[runs++] = segs;
+    for (int z = 0; z < pl.S; ++z) {
+      if (bp.mode == 3) p.run_start[runs++] = segs;
+      HessSeg& g = p.seg[segs++];
+      g.map = b;
+      g.tok0 = z * pl.tokens_per_slice;
+      g.tok_end = (int)std::min<int64_t>(n[b], g.tok0 + (int64_t)pl.tokens_per_slice);
+      g.part = bp.mode == 1 ? -1 : part;
+      g.add = bp.mode == 1 || (bp.mode == 2 && z > 0);
+      if (bp.mode == 3) ++part;
+    }
+    if (bp.mode == 2) ++part;
+  }
+  p.run_start[runs] = segs;
+  if (part_start) part_start[count] = part;
+  return launch_pair(p, runs, s);
+}
+
 // H (lower blocks) += X^T X.  `reduce` is called by the caller when S > 1 (slice buffers -> H).
 int launch_hessian_umma(const HessPlan& pl, const void* X, int x_dtype, int64_t n, int64_t K, float* H, void* ws,
                         int32_t* status, cudaStream_t s) {
@@ -623,11 +778,9 @@ int launch_hessian_umma(const HessPlan& pl, const void* X, int x_dtype, int64_t 
     __nv_bfloat16* P0 = (__nv_bfloat16*)w;
     __nv_bfloat16* P1 = (__nv_bfloat16*)(w + pl.plane_bytes);
     w += 2 * pl.plane_bytes;
-    const int64_t total4 = n * K / 4;
-    const int blocks = (int)std::min<int64_t>(cdiv(total4, 256), (int64_t)sm_count() * 16);
-    prefer_shared_carveout<split_bf16_kernel<float>>();
-    split_bf16_kernel<float><<<blocks, 256, 0, s>>>((const float*)X, P0, P1, total4);
-    JGQ_LAUNCHED();
+    SplitParams sp;
+    sp.X[0] = (const float*)X; sp.P0[0] = P0; sp.P1[0] = P1; sp.total4[0] = n * K / 4;
+    split_planes(sp, 1, n * K / 4, s);
     plane0 = P0;
     plane1 = P1;
   }
@@ -644,33 +797,22 @@ int launch_hessian_umma(const HessPlan& pl, const void* X, int x_dtype, int64_t 
   p.out = pl.S > 1 ? part : H;
   p.slice_stride = pl.S > 1 ? K * K : 0;
   p.status = status;
-  // Test hook for the bounded waits: with JGQ_TEST_WITHHOLD_COMMIT set (read at every launch) the MMA warp keeps its
-  // first "chain finished" signal to itself; the waits of every role then run out their budget, the kernel returns
-  // without writing H and reports JGQ_STATUS_TIMEOUT.  Nothing faults and nothing spins without a limit.
-  p.withhold_first_chain = getenv("JGQ_TEST_WITHHOLD_COMMIT") ? 1 : 0;
+  p.withhold_first_chain = getenv("JGQ_TEST_WITHHOLD_COMMIT") ? 1 : 0;      // test hook, see launch_pair
   if (pl.panel == 256) {
-    struct PairAttrTag {};
-    once_per_device<PairAttrTag>([]() {
-      cudaFuncSetAttribute(hessian_pair_kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 0);
-      cudaGetLastError();
-      return (int)cudaFuncSetAttribute(hessian_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       HP_RING_BYTES + HT_BAR_BYTES);
-    });
-    cudaLaunchConfig_t cfg;
-    memset(&cfg, 0, sizeof(cfg));
-    cfg.gridDim = dim3((unsigned)(2 * pl.nseg * pl.S));
-    cfg.blockDim = dim3(HT_THREADS);
-    cfg.dynamicSmemBytes = HP_RING_BYTES + HT_BAR_BYTES;
-    cfg.stream = s;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = 2; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    const cudaError_t e = cudaLaunchKernelEx(&cfg, hessian_pair_kernel, m0, m1, p);
-    note_launches(1);
-    if (e != cudaSuccess) { cudaGetLastError(); return fail(JGQ_ERR_CUDA, "hessian_pair: %s", cudaGetErrorString(e)); }
-    return JGQ_OK;
+    HessPairParams pp;
+    memset(&pp, 0, sizeof(pp));
+    pp.maps[0] = m0; pp.maps[1] = m1;
+    pp.K = (int)K; pp.planes = pl.planes; pp.fmt = p.fmt; pp.nseg = pl.nseg;
+    pp.H = H; pp.parts = part; pp.part_stride = K * K; pp.status = status;
+    for (int z = 0; z < pl.S; ++z) {
+      pp.run_start[z] = z;
+      HessSeg& g = pp.seg[z];
+      g.map = 0; g.tok0 = z * pl.tokens_per_slice;
+      g.tok_end = (int)std::min<int64_t>(n, g.tok0 + (int64_t)pl.tokens_per_slice);
+      g.part = pl.S > 1 ? z : -1; g.add = pl.S == 1;
+    }
+    pp.run_start[pl.S] = pl.S;
+    return launch_pair(pp, pl.S, s);
   }
   struct SmemAttrTag {};
   once_per_device<SmemAttrTag>([]() {

@@ -9,6 +9,8 @@ libjgq.so; there is no PyTorch or CPU implementation behind these functions.
 """
 from __future__ import annotations
 
+import ctypes
+
 import numpy as np
 import torch
 
@@ -234,9 +236,43 @@ def _chunk_rows(n, K, dt):
     return max(1, rows)
 
 
+_MAX_BATCHES = 16        # batches of one jgq_hessian_accum_batches call that share a launch
+
+
 def _accumulate_raw(xs, H=None, status=None):
-    """H (K x K fp32, lower triangle) += sum over batches of X^T X; returns (H, n)."""
+    """H (K x K fp32, lower triangle) += sum over batches of X^T X; returns (H, n).
+
+    Batches are handed to the library in order, several to a call as long as the scratch of the call stays below
+    _MAX_HESSIAN_SCRATCH (the same result as one by one)."""
     n_total = 0
+    group = []               # 2-D contiguous batches of one dtype and width, waiting to be enqueued
+    held = 0                 # bytes of them that exist only for this call (copies of host batches, conversions)
+
+    def flush():
+        if not group:
+            return
+        dt, K = _DT[group[0].dtype], group[0].shape[1]
+        if len(group) == 1:
+            m = group[0].shape[0]
+            need = lib.jgq_hessian_workspace_bytes(m, K, dt)
+            ws = _workspace_for(need) if need else None
+            check(lib.jgq_hessian_accum(group[0].data_ptr(), dt, m, K, H.data_ptr(), _ptr(ws), need, _ptr(status), _stream()))
+            group.clear()
+            return
+        rows = (ctypes.c_int64 * len(group))(*(b.shape[0] for b in group))
+        need = lib.jgq_hessian_batches_workspace_bytes(rows, len(group), K, dt)
+        if need > _MAX_HESSIAN_SCRATCH:          # two halves, each in turn
+            rest = group[len(group) // 2:]
+            del group[len(group) // 2:]
+            flush()
+            group.extend(rest)
+            flush()
+            return
+        ptrs = (ctypes.c_void_p * len(group))(*(b.data_ptr() for b in group))
+        ws = _workspace_for(need) if need else None
+        check(lib.jgq_hessian_accum_batches(ptrs, rows, len(group), dt, K, H.data_ptr(), _ptr(ws), need, _ptr(status), _stream()))
+        group.clear()
+
     for batch in _merge_adjacent(list(xs)):
         b = _to_dev(batch)
         if b.dtype not in _DT:
@@ -248,15 +284,20 @@ def _accumulate_raw(xs, H=None, status=None):
         if H is None:
             H = _tmp('H', (K, K), torch.float32, zero=True)
         n = b.shape[0]
+        if not (isinstance(batch, torch.Tensor) and batch.is_cuda and batch.untyped_storage().data_ptr() == b.untyped_storage().data_ptr()):
+            size = b.numel() * b.element_size()
+            if held + size > _MAX_HESSIAN_SCRATCH:
+                flush()
+                held = 0
+            held += size
         rows = _chunk_rows(n, K, _DT[b.dtype])
         for r0 in range(0, n, rows):
-            chunk = b[r0:r0 + rows]
-            m = chunk.shape[0]
-            need = lib.jgq_hessian_workspace_bytes(m, K, _DT[chunk.dtype])
-            ws = _workspace_for(need) if need else None
-            check(lib.jgq_hessian_accum(chunk.data_ptr(), _DT[chunk.dtype], m, K, H.data_ptr(),
-                                        _ptr(ws), need, _ptr(status), _stream()))
+            chunk = b if rows >= n else b[r0:r0 + rows]
+            if group and (len(group) == _MAX_BATCHES or group[0].dtype != chunk.dtype or group[0].shape[1] != K):
+                flush()
+            group.append(chunk)
         n_total += n
+    flush()
     return H, n_total
 
 

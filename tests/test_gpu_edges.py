@@ -101,3 +101,23 @@ def test_quantize_loop_values_outside_the_fast_quotients(gg):
     got = Qd.cpu().numpy()
     ok = np.isfinite(Q) & (np.arange(N) != 6)[None, :]                  # behind the infinite weight clip(NaN) is the host's choice
     assert np.array_equal(got[ok], Q[ok])
+
+
+@pytest.mark.parametrize('K,ns,dtype', [(512, (600, 1333, 2048, 777), torch.float32), (768, (1024,) * 4, torch.float32),
+                                        (1800, (1500, 4096, 5000), torch.bfloat16), (1024, (512, 100, 700), torch.float32),
+                                        (1032, (2048,) * 5, torch.float16), (2048, (1024,) * 17, torch.bfloat16),
+                                        (3072, (4096,) * 3, torch.float32), (256, (1000, 600), torch.float32),
+                                        (300, (700, 40), torch.float16)])
+def test_hessian_of_separate_batches_equals_one_by_one(gg, K, ns, dtype):
+    """Batches that share a launch (tile by tile, batch by batch or slice by slice, whichever the plan takes), batches too
+    small or too odd for it, and more than fit one call: the bits of one call per batch."""
+    g = torch.Generator(device='cuda').manual_seed(K + len(ns))
+    xs = [(torch.randn((n, K), generator=g, device='cuda') + 0.3).to(dtype) for n in ns]
+    together, n = gg._accumulate_raw(xs)
+    assert n == sum(ns)
+    H = torch.zeros((K, K), device='cuda')
+    for x in xs:
+        gg._accumulate_raw([x], H=H)
+    assert torch.equal(together.tril(), H.tril())
+    ref = sum(x.double().T @ x.double() for x in xs)
+    assert ((together.double() - ref).tril().norm() / ref.tril().norm()).item() < 3e-6
