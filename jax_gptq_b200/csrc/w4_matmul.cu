@@ -263,7 +263,7 @@ static int launch_fwd(const void* x, const uint8_t* packed, const void* zero, co
 constexpr int64_t kStreamRows = 16;          // token rows of one pass of the streaming kernel
 constexpr int64_t kStreamPassesMaxM = 32;    // two passes (120 us at 8192 x 28672) still beat the tensor-path kernel (128 us at M = 64)
 
-static int w4_path_override() {        // JGQ_W4_PATH=direct: direct-load decode kernel; =mma: no tcgen05 either; =stream: no f16 decode kernel
+static int w4_path_override() {        // JGQ_W4_PATH=direct: direct-load decode kernel; =mma: no tcgen05 either; =stream: no decode kernel
   static const int v = []() {
     const char* e = getenv("JGQ_W4_PATH");
     return !e ? 0 : !strcmp(e, "direct") ? 1 : !strcmp(e, "mma") ? 2 : !strcmp(e, "stream") ? 3 : 0;
@@ -281,7 +281,9 @@ using namespace jgq;
 
 namespace jgq {
 
-// Scratch bytes of the forward matmul for one activation dtype (x_dtype < 0: the largest over all dtypes).
+// Scratch bytes of the forward matmul for one activation dtype (x_dtype < 0: the largest over all dtypes): what a
+// call is refused without.  The decode kernel for other types than f16, or more than 16 rows, may want more than
+// that: it is taken when the workspace holds it (w4_forward_best).
 static size_t w4_forward_need(int64_t M, int64_t N, int64_t K, int x_dtype) {
   if (M <= 0 || N <= 0 || K <= 0) return 0;
   const FwdPlan p = plan_fwd(M, N, K);
@@ -300,9 +302,19 @@ static size_t w4_forward_need(int64_t M, int64_t N, int64_t K, int x_dtype) {
   const StreamPlan sp = plan_w4_stream(std::min<int64_t>(M, kStreamPassesMaxM) > kStreamRows ? kStreamRows : M, N, K);
   if (sp.use && M <= kStreamPassesMaxM) bytes = std::max(bytes, kTicketBytes + sp.part_bytes);
   if (x_dtype < 0 || x_dtype == JGQ_F16) {
-    const GemvPlan gp = plan_w4_gemv(M, N, K);
-    if (gp.use) bytes = std::max(bytes, gp.ws_bytes);
+    const GemvPlan gp = plan_w4_gemv(std::min<int64_t>(M, kStreamRows), N, K, JGQ_F16);
+    if (gp.use && M <= kStreamRows) bytes = std::max(bytes, gp.ws_bytes);
   }
+  return bytes;
+}
+
+static size_t w4_forward_best(int64_t M, int64_t N, int64_t K) {
+  size_t bytes = w4_forward_need(M, N, K, -1);
+  for (int dt : {JGQ_F32, JGQ_F16, JGQ_BF16})
+    for (int64_t rows : {M, std::min<int64_t>(M, kStreamRows)}) {
+      const GemvPlan gp = plan_w4_gemv(rows, N, K, dt);
+      if (M <= kStreamPassesMaxM && gp.use) bytes = std::max(bytes, gp.ws_bytes);
+    }
   return bytes;
 }
 
@@ -331,7 +343,7 @@ static int w4_validate(const void* x, int x_dtype, const uint8_t* packed, const 
 // (possibly smaller) amount its own dtype needs.
 extern "C" size_t jgq_w4_matmul_workspace_bytes(int64_t M, int64_t N, int64_t K, int transpose_b) {
   if (transpose_b) return (M > 0 && N > 0 && K > 0) ? w4_tb_workspace_bytes(M, N) : 0;
-  return w4_forward_need(M, N, K, -1);
+  return (M > 0 && N > 0 && K > 0) ? w4_forward_best(M, N, K) : 0;
 }
 
 extern "C" int jgq_w4_matmul(const void* x, int x_dtype, const uint8_t* packed,
@@ -354,10 +366,25 @@ extern "C" int jgq_w4_matmul(const void* x, int x_dtype, const uint8_t* packed,
   const size_t need = w4_forward_need(M, N, K, x_dtype);
   JGQ_REQUIRE(ws && ws_bytes >= need, JGQ_ERR_WORKSPACE, "w4_matmul: workspace %zu < %zu bytes", ws_bytes, need);
   JGQ_REQUIRE(aligned(ws, 256), JGQ_ERR_ALIGN, "w4_matmul: workspace must be 256-byte aligned");
-  if (w4_path_override() == 0 && x_dtype == JGQ_F16) {
-    const GemvPlan gp = plan_w4_gemv(M, N, K);
-    if (gp.use && aligned(packed, 16) && aligned(x, 16) && aligned(out, 8))
-      return launch_w4_gemv(gp, x, packed, zero, scale, zs_dtype, out, M, N, K, ws, settled, s);
+  // Decode sizes: one pass over the weights for all rows, or one per 16 rows (fp32 activations beyond 16; a
+  // workspace too small for the slices of 32).  Above 32 rows the tensor-path kernel is the faster one.
+  if (w4_path_override() == 0 && M <= kStreamPassesMaxM && aligned(packed, 16) && aligned(x, 16) && aligned(out, x_dtype == JGQ_F32 ? 16 : 8)) {
+    const size_t elt = dtype_size(x_dtype);
+    for (int64_t step : {M, std::min<int64_t>(M, kStreamRows)}) {
+      bool ok = true;
+      for (int64_t r0 = 0; r0 < M && ok; r0 += step) {
+        const GemvPlan gp = plan_w4_gemv(std::min<int64_t>(step, M - r0), N, K, x_dtype);
+        ok = gp.use && gp.ws_bytes <= ws_bytes;
+      }
+      if (!ok) continue;
+      for (int64_t r0 = 0; r0 < M; r0 += step) {
+        const int64_t rows = std::min<int64_t>(step, M - r0);
+        const int rc = launch_w4_gemv(plan_w4_gemv(rows, N, K, x_dtype), (const char*)x + (size_t)r0 * K * elt, x_dtype, packed, zero,
+                                      scale, zs_dtype, (char*)out + (size_t)r0 * N * elt, rows, N, K, ws, settled, s);
+        if (rc) return rc;
+      }
+      return JGQ_OK;
+    }
   }
   if (w4_path_override() == 0 || w4_path_override() == 3) {
     const StreamPlan sp = plan_w4_stream(M, N, K);

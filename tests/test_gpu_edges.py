@@ -121,3 +121,55 @@ def test_hessian_of_separate_batches_equals_one_by_one(gg, K, ns, dtype):
     assert torch.equal(together.tril(), H.tril())
     ref = sum(x.double().T @ x.double() for x in xs)
     assert ((together.double() - ref).tril().norm() / ref.tril().norm()).item() < 3e-6
+
+
+@pytest.mark.parametrize('M', [1, 2, 3, 5, 8, 9, 16, 17, 31, 32, 33])
+@pytest.mark.parametrize('dtype', [torch.float16, torch.bfloat16, torch.float32])
+@pytest.mark.parametrize('K,N', [(8, 16), (136, 48), (3080, 144), (768, 2304)])
+def test_matmul_decode_rows_types_and_ragged_edges(gg, M, dtype, K, N):
+    """Token counts around the groups of eight, channel groups that are not full, contraction ranges that end inside a
+    box.  Against the dequantized product in fp64: the output's rounding (2^-11, 2^-8, or the two bf16 planes' 2^-17 with
+    fp32 sums over at most 3080 terms), in the 2-norm."""
+    from jax_gptq_b200 import quantized_matmul, QuantizedMatrix
+    g = torch.Generator(device='cuda').manual_seed(1000 * M + K + N)
+    packed = torch.randint(0, 256, (K // 2, N), generator=g, device='cuda', dtype=torch.uint8)
+    zs = torch.float32 if M % 2 else torch.float16
+    scale = (0.001 + 0.019 * torch.rand(N, generator=g, device='cuda')).to(zs)
+    zero = torch.randint(0, 16, (N,), generator=g, device='cuda').to(zs)
+    x = torch.randn((M, K), generator=g, device='cuda').to(dtype)
+    dense = (torch.stack([packed & 15, packed >> 4], 1).reshape(K, N).double() - zero.double()) * scale.double()
+    want = x.double() @ dense
+    bound = {torch.float16: 2.0 ** -11, torch.bfloat16: 2.0 ** -8, torch.float32: 2e-5}[dtype]
+    first = None
+    for _ in range(3):                                  # the later calls fetch weights early
+        got = quantized_matmul(x, QuantizedMatrix(packed, zero, scale))
+        assert ((got.double() - want).norm() / want.norm()).item() <= bound
+        assert first is None or torch.equal(got, first)
+        first = got
+
+
+@pytest.mark.parametrize('M,dtype', [(24, torch.float16), (32, torch.bfloat16), (12, torch.float32), (20, torch.float32)])
+def test_matmul_with_the_smallest_workspace_it_accepts(gg, M, dtype):
+    """The slices of 32 rows are larger than what a call is refused without; with a smaller workspace it takes two passes."""
+    from jax_gptq_b200 import _lib
+    lib = _lib.lib
+    N, K = 2048, 8192
+    g = torch.Generator(device='cuda').manual_seed(M)
+    packed = torch.randint(0, 256, (K // 2, N), generator=g, device='cuda', dtype=torch.uint8)
+    scale, zero = torch.rand(N, generator=g, device='cuda') * 0.01, torch.full((N,), 8.0, device='cuda')
+    x = torch.randn((M, K), generator=g, device='cuda').to(dtype)
+    full = lib.jgq_w4_matmul_workspace_bytes(M, N, K, 0)
+    outs = []
+    ws = torch.zeros(full, dtype=torch.uint8, device='cuda')
+    for nbytes in (full, full // 2, full // 4, full // 8):
+        out = torch.full((M, N), float('nan'), dtype=dtype, device='cuda')
+        rc = lib.jgq_w4_matmul(x.data_ptr(), gg._DT[dtype], packed.data_ptr(), zero.data_ptr(), scale.data_ptr(), _lib.F32,
+                               out.data_ptr(), M, N, K, 0, ws.data_ptr(), nbytes, gg._stream())
+        if rc == -3:
+            continue
+        assert rc == 0
+        outs.append(out)
+    want = x.double() @ ((torch.stack([packed & 15, packed >> 4], 1).reshape(K, N).double() - 8) * scale.double())
+    for out in outs:
+        assert ((out.double() - want).norm() / want.norm()).item() <= {torch.float16: 2.0 ** -11, torch.bfloat16: 2.0 ** -8, torch.float32: 2e-5}[dtype]
+    assert int(ws[:16384].sum()) == 0                    # the tickets are back at zero
