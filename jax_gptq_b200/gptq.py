@@ -69,7 +69,8 @@ _ws_cache = {}
 def _workspace(nbytes, zeroed=False, tag='ws'):
     """Per (device, stream) scratch buffer, grown on demand.  `zeroed` buffers are
     created with zeros and handed only to kernels that restore the zeros."""
-    key = (torch.cuda.current_device(), _stream(), tag)
+    dev = torch.cuda.current_device()
+    key = (dev, torch._C._cuda_getCurrentRawStream(dev), tag)
     buf = _ws_cache.get(key)
     if buf is None or buf.numel() < nbytes:
         size = max(int(nbytes), 1 << 20)

@@ -173,3 +173,43 @@ def test_matmul_with_the_smallest_workspace_it_accepts(gg, M, dtype):
     for out in outs:
         assert ((out.double() - want).norm() / want.norm()).item() <= {torch.float16: 2.0 ** -11, torch.bfloat16: 2.0 ** -8, torch.float32: 2e-5}[dtype]
     assert int(ws[:16384].sum()) == 0                    # the tickets are back at zero
+
+
+def _some_matrix(K=256, N=128):
+    from jax_gptq_b200 import QuantizedMatrix
+    g = torch.Generator(device='cuda').manual_seed(5)
+    return QuantizedMatrix(torch.randint(0, 256, (K // 2, N), generator=g, device='cuda', dtype=torch.uint8),
+                           torch.full((N,), 8.0, device='cuda'), torch.rand(N, generator=g, device='cuda') * 0.01)
+
+
+def test_matmul_outside_and_inside_autograd(gg):
+    """A product that nothing differentiates is launched directly; with gradients (of the input, or recorded for the
+    scales), under forward mode and under a functorch transform it still goes through the autograd function."""
+    from jax_gptq_b200 import quantized_matmul
+    qm = _some_matrix()
+    x = torch.randn((2, 3, 256), device='cuda')
+    plain = quantized_matmul(x, qm)
+    assert plain.shape == (2, 3, 128) and not plain.requires_grad
+    xg = x.clone().requires_grad_()
+    y = quantized_matmul(xg, qm)
+    assert y.requires_grad and torch.equal(y.detach(), plain)
+    y.sum().backward()
+    assert torch.equal(xg.grad, quantized_matmul(torch.ones_like(y), qm, transpose_b=True))
+    with torch.no_grad():
+        assert not quantized_matmul(xg, qm).requires_grad
+    qm.scale.requires_grad_()
+    assert quantized_matmul(x, qm).requires_grad
+    qm.scale.requires_grad_(False)
+    with torch.autograd.forward_ad.dual_level():
+        dual = torch.autograd.forward_ad.make_dual(x, torch.ones_like(x))
+        with pytest.raises(RuntimeError):
+            quantized_matmul(dual, qm)
+    with pytest.raises(RuntimeError):
+        torch.func.vmap(lambda r: quantized_matmul(r, qm))(x)
+    assert torch.equal(quantized_matmul(x.transpose(0, 1), qm), plain.transpose(0, 1))
+    assert torch.equal(quantized_matmul(torch.nn.Parameter(x, requires_grad=False), qm), plain)
+    with pytest.raises(ValueError):
+        quantized_matmul(x[0, 0], qm)
+    traced = torch.jit.trace(lambda t: quantized_matmul(t, qm), (x,), check_trace=False)
+    other = torch.randn_like(x)
+    assert torch.equal(traced(other), quantized_matmul(other, qm))
