@@ -146,4 +146,86 @@ __device__ __forceinline__ void w4_step(float (&acc)[NTOK][8][4], float (&accx)[
   }
 }
 
+template <typename T>
+__global__ void xsum_kernel(const T* __restrict__ x, float* __restrict__ xsum, int64_t K) {
+  __shared__ float part[8];
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  const int64_t m = blockIdx.x;
+  float s = 0.f;
+  for (int64_t k = threadIdx.x; k < K; k += blockDim.x) s += to_f32<T>(x[m * K + k]);
+  for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+  if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = s;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    float t = 0.f;
+    for (int w = 0; w < (int)(blockDim.x >> 5); ++w) t += part[w];
+    xsum[m] = t;
+  }
+}
+
+// sum over k of the two bf16 planes of a split fp32 activation row: exactly what the MMAs see, so that
+// the offset of the expanded codes cancels exactly in the epilogue
+static __global__ void xsum_planes_kernel(const __nv_bfloat16* __restrict__ P0, const __nv_bfloat16* __restrict__ P1,
+                                   float* __restrict__ xsum, int64_t K) {
+  __shared__ float part[8];
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  const int64_t m = blockIdx.x;
+  float s = 0.f;
+  for (int64_t k = threadIdx.x; k < K; k += blockDim.x)
+    s += __bfloat162float(P0[m * K + k]) + __bfloat162float(P1[m * K + k]);
+  for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+  if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = s;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    float t = 0.f;
+    for (int w = 0; w < (int)(blockDim.x >> 5); ++w) t += part[w];
+    xsum[m] = t;
+  }
+}
+
+static __global__ void split_x_bf16_kernel(const float* __restrict__ X, __nv_bfloat16* __restrict__ P0,
+                                    __nv_bfloat16* __restrict__ P1, int64_t total) {
+  for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < total;
+       t += (int64_t)gridDim.x * blockDim.x) {
+    const float v = X[t];
+    const __nv_bfloat16 h = __float2bfloat16_rn(v);
+    P0[t] = h;
+    P1[t] = __float2bfloat16_rn(v - __bfloat162float(h));
+  }
+}
+
+// 8 codes of one 32-bit word (4 channels x {k even, k odd}) -> four 2-channel registers.
+// e02 / e13: k even, channels (0,2) / (1,3);  o02 / o13: k odd.
+// The integer / logic pipe is the scarce one (half rate), so the constants come from kernel
+// parameters (a mask and an exponent pattern as two immediates would cost two logic instructions
+// per register) and the magic offset is removed on the FMA pipe:
+//   f16:  0x6400 | c = 1024 + c -> subtract 1024;   0x6400 | c << 4 = 1024 + 16 c -> * 1/16 - 64
+//   bf16: 0x4300 | c = 128 + c  -> subtract 128 (a nibble does not fit above bit 3 of a bf16 mantissa
+//         without reaching the exponent, so the high nibbles are shifted down)
+template <int FMT>
+__device__ __forceinline__ void expand_word(uint32_t w, uint32_t mask_lo, uint32_t mask_hi, uint32_t magic,
+                                            uint32_t& e02, uint32_t& e13, uint32_t& o02, uint32_t& o13) {
+  if (FMT == 0) {
+    const uint32_t w8 = w >> 8;
+    uint32_t a = (w & mask_lo) | magic, b = (w8 & mask_lo) | magic;
+    uint32_t c = (w & mask_hi) | magic, d = (w8 & mask_hi) | magic;
+    const __half2 k1024 = __half2half2(__float2half_rn(1024.f));
+    const __half2 k16th = __half2half2(__float2half_rn(0.0625f)), k64 = __half2half2(__float2half_rn(-64.f));
+    __half2 ra = __hsub2(*reinterpret_cast<__half2*>(&a), k1024), rb = __hsub2(*reinterpret_cast<__half2*>(&b), k1024);
+    __half2 rc = __hfma2(*reinterpret_cast<__half2*>(&c), k16th, k64), rd = __hfma2(*reinterpret_cast<__half2*>(&d), k16th, k64);
+    e02 = *reinterpret_cast<uint32_t*>(&ra); e13 = *reinterpret_cast<uint32_t*>(&rb);
+    o02 = *reinterpret_cast<uint32_t*>(&rc); o13 = *reinterpret_cast<uint32_t*>(&rd);
+  } else {
+    uint32_t a = (w & mask_lo) | magic, b = ((w >> 8) & mask_lo) | magic;
+    uint32_t c = ((w >> 4) & mask_lo) | magic, d = ((w >> 12) & mask_lo) | magic;
+    const __nv_bfloat162 k128 = __float2bfloat162_rn(128.f);
+    __nv_bfloat162 ra = __hsub2(*reinterpret_cast<__nv_bfloat162*>(&a), k128);
+    __nv_bfloat162 rb = __hsub2(*reinterpret_cast<__nv_bfloat162*>(&b), k128);
+    __nv_bfloat162 rc = __hsub2(*reinterpret_cast<__nv_bfloat162*>(&c), k128);
+    __nv_bfloat162 rd = __hsub2(*reinterpret_cast<__nv_bfloat162*>(&d), k128);
+    e02 = *reinterpret_cast<uint32_t*>(&ra); e13 = *reinterpret_cast<uint32_t*>(&rb);
+    o02 = *reinterpret_cast<uint32_t*>(&rc); o13 = *reinterpret_cast<uint32_t*>(&rd);
+  }
+}
+
 }  // namespace jgq

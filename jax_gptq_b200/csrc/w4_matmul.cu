@@ -308,12 +308,40 @@ static size_t w4_forward_need(int64_t M, int64_t N, int64_t K, int x_dtype) {
   return bytes;
 }
 
+// Pair kernel or single-CTA kernel, for forward products of more than 32 rows both can run.  Estimates in us, fitted to
+// the GPU time of 9 row counts from 33 to 2048 on seven weight shapes from 768 x 2304 to 8192 x 28672:
+//   single CTA   13 per wave, 0.3 to 0.7 per stage (more with the tile's tokens), 9 per slice of a split contraction and 128
+//                tokens for the slices' exchange;
+//   pair         7 per wave of 74, 0.45 per stage with one block of 256 tokens, 0.7 with two.
+// The single-CTA kernel keeps few rows on long contractions (64 rows, K = 11008, N = 4096: 76 against 82 us; 128 rows of
+// fp32: 87 against 133); more than 256 rows of 16-bit activations always go to the pairs (2048 rows, 4096 x 11008: 293
+// against 176 us).  The transposed product takes the pairs whenever they can run (33 rows, 4096 x 4096: 108 against
+// 53 us; 2048 rows, 11008 x 4096: 894 against 276).
+static PairPlan w4_pair_choice(int64_t M, int64_t N, int64_t K, int x_dtype, int transpose_b) {
+  const int ov = w4_path_override();
+  PairPlan pp = plan_w4_pair(M, N, K, x_dtype, transpose_b);
+  if (!pp.use || ov != 0 || transpose_b) { pp.use = pp.use && ov == 0; return pp; }
+  if (M <= kStreamPassesMaxM) { pp.use = 0; return pp; }
+  if (pp.planes == 1 && M > 256) return pp;
+  const UmmaPlan up = plan_w4_umma(M, N, K, x_dtype);
+  if (!up.use) return pp;
+  const int sms = sm_count();
+  const double pair = (double)cdiv(pp.units, std::max(1, sms / 2)) * ((pp.planes == 2 ? 0.7 : 0.45) * (double)cdiv(pp.depth, 64) + 7.0);
+  const double stage = up.planes == 2 ? 0.35 + 0.0022 * up.NT : 0.3 + 0.0016 * up.NT;
+  const double single = (double)cdiv((int64_t)up.ncg * up.mtiles * up.ksplit, sms) * (stage * up.stages_per_split + 13.0) +
+                        (up.ksplit > 1 ? 9.0 / 128.0 * up.NT * up.ksplit : 0.0);
+  pp.use = pair + 8.0 < 0.93 * (single + 10.0);
+  return pp;
+}
+
 static size_t w4_forward_best(int64_t M, int64_t N, int64_t K) {
   size_t bytes = w4_forward_need(M, N, K, -1);
   for (int dt : {JGQ_F32, JGQ_F16, JGQ_BF16})
     for (int64_t rows : {M, std::min<int64_t>(M, kStreamRows)}) {
       const GemvPlan gp = plan_w4_gemv(rows, N, K, dt);
       if (M <= kStreamPassesMaxM && gp.use) bytes = std::max(bytes, gp.ws_bytes);
+      const PairPlan pp = w4_pair_choice(M, N, K, dt, 0);
+      if (pp.use) bytes = std::max(bytes, pp.ws_bytes);
     }
   return bytes;
 }
@@ -342,7 +370,11 @@ static int w4_validate(const void* x, int x_dtype, const uint8_t* packed, const 
 // The size returned covers every activation dtype; a call is accepted with the
 // (possibly smaller) amount its own dtype needs.
 extern "C" size_t jgq_w4_matmul_workspace_bytes(int64_t M, int64_t N, int64_t K, int transpose_b) {
-  if (transpose_b) return (M > 0 && N > 0 && K > 0) ? w4_tb_workspace_bytes(M, N) : 0;
+  if (transpose_b) {
+    if (M <= 0 || N <= 0 || K <= 0) return 0;
+    const PairPlan pp = w4_pair_choice(M, N, K, JGQ_F32, 1);
+    return std::max(w4_tb_workspace_bytes(M, N), pp.use ? pp.ws_bytes : 0);
+  }
   return (M > 0 && N > 0 && K > 0) ? w4_forward_best(M, N, K) : 0;
 }
 
@@ -360,6 +392,9 @@ extern "C" int jgq_w4_matmul(const void* x, int x_dtype, const uint8_t* packed,
     const size_t need_tb = w4_tb_workspace_bytes(M, N);
     JGQ_REQUIRE(ws && ws_bytes >= need_tb, JGQ_ERR_WORKSPACE, "w4_matmul: workspace %zu < %zu bytes", ws_bytes, need_tb);
     JGQ_REQUIRE(aligned(ws, 256), JGQ_ERR_ALIGN, "w4_matmul: workspace must be 256-byte aligned");
+    const PairPlan pp = w4_pair_choice(M, N, K, x_dtype, 1);
+    if (pp.use && pp.ws_bytes <= ws_bytes && aligned(packed, 16))
+      return launch_w4_pair(pp, x, x_dtype, packed, zero, scale, zs_dtype, out, M, N, K, 1, ws, s);
     return launch_w4_tb(x, x_dtype, packed, zero, scale, zs_dtype, out, M, N, K, ws, s);
   }
   JGQ_REQUIRE(aligned(x, 8), JGQ_ERR_ALIGN, "w4_matmul: x must be 8-byte aligned");
@@ -410,6 +445,9 @@ extern "C" int jgq_w4_matmul(const void* x, int x_dtype, const uint8_t* packed,
     }
   }
   if (!w4_force_mma_sync()) {
+    const PairPlan pp = w4_pair_choice(M, N, K, x_dtype, 0);
+    if (pp.use && pp.ws_bytes <= ws_bytes && aligned(x, 16) && aligned(packed, 16))
+      return launch_w4_pair(pp, x, x_dtype, packed, zero, scale, zs_dtype, out, M, N, K, 0, ws, s);
     const UmmaPlan up = plan_w4_umma(M, N, K, x_dtype);
     if (M > 16 && up.use && aligned(x, 16) && aligned(packed, 16) && aligned(out, 4))
       return launch_w4_umma(up, x, x_dtype, packed, zero, scale, zs_dtype, out, M, N, K, ws, s);

@@ -33,6 +33,15 @@ size_t w4_tb_workspace_bytes(int64_t M, int64_t N);
 int launch_w4_tb(const void* x, int x_dtype, const uint8_t* packed, const void* zero, const void* scale, int zs_dtype,
                  void* out, int64_t M, int64_t N, int64_t K, void* ws, cudaStream_t s);
 
+// CTA-pair kernel for many tokens, forward and transposed (w4_pair.cu); use: it can run (the dispatcher chooses)
+struct PairPlan {
+  int use; int planes; int tile; int rows; int depth; int nrp; int units; int64_t Np;
+  size_t plane_bytes; size_t ws_bytes;
+};
+PairPlan plan_w4_pair(int64_t M, int64_t N, int64_t K, int x_dtype, int transpose_b);
+int launch_w4_pair(const PairPlan& pl, const void* x, int x_dtype, const uint8_t* packed, const void* zero, const void* scale,
+                   int zs_dtype, void* out, int64_t M, int64_t N, int64_t K, int transpose_b, void* ws, cudaStream_t s);
+
 // decode kernel, M <= 32, fp32 activations M <= 16 (w4_gemv.cu)
 struct GemvPlan {
   int use; int nt; int rows; int ncg; int spc; int64_t S; int G; int maxc;

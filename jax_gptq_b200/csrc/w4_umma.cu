@@ -56,86 +56,6 @@ struct UmmaParams {
   uint32_t emask_lo, emask_hi, emagic;   // nibble expansion: (bits & mask) | emagic
 };
 
-template <typename T>
-__global__ void xsum_kernel(const T* __restrict__ x, float* __restrict__ xsum, int64_t K) {
-  __shared__ float part[8];
-  const int64_t m = blockIdx.x;
-  float s = 0.f;
-  for (int64_t k = threadIdx.x; k < K; k += blockDim.x) s += to_f32<T>(x[m * K + k]);
-  for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-  if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = s;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    float t = 0.f;
-    for (int w = 0; w < (int)(blockDim.x >> 5); ++w) t += part[w];
-    xsum[m] = t;
-  }
-}
-
-// sum over k of the two bf16 planes of a split fp32 activation row: exactly what the MMAs see, so that
-// the offset of the expanded codes cancels exactly in the epilogue
-__global__ void xsum_planes_kernel(const __nv_bfloat16* __restrict__ P0, const __nv_bfloat16* __restrict__ P1,
-                                   float* __restrict__ xsum, int64_t K) {
-  __shared__ float part[8];
-  const int64_t m = blockIdx.x;
-  float s = 0.f;
-  for (int64_t k = threadIdx.x; k < K; k += blockDim.x)
-    s += __bfloat162float(P0[m * K + k]) + __bfloat162float(P1[m * K + k]);
-  for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-  if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = s;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    float t = 0.f;
-    for (int w = 0; w < (int)(blockDim.x >> 5); ++w) t += part[w];
-    xsum[m] = t;
-  }
-}
-
-__global__ void split_x_bf16_kernel(const float* __restrict__ X, __nv_bfloat16* __restrict__ P0,
-                                    __nv_bfloat16* __restrict__ P1, int64_t total) {
-  for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < total;
-       t += (int64_t)gridDim.x * blockDim.x) {
-    const float v = X[t];
-    const __nv_bfloat16 h = __float2bfloat16_rn(v);
-    P0[t] = h;
-    P1[t] = __float2bfloat16_rn(v - __bfloat162float(h));
-  }
-}
-
-// 8 codes of one 32-bit word (4 channels x {k even, k odd}) -> four 2-channel registers.
-// e02 / e13: k even, channels (0,2) / (1,3);  o02 / o13: k odd.
-// The integer / logic pipe is the scarce one (half rate), so the constants come from kernel
-// parameters (a mask and an exponent pattern as two immediates would cost two logic instructions
-// per register) and the magic offset is removed on the FMA pipe:
-//   f16:  0x6400 | c = 1024 + c -> subtract 1024;   0x6400 | c << 4 = 1024 + 16 c -> * 1/16 - 64
-//   bf16: 0x4300 | c = 128 + c  -> subtract 128 (a nibble does not fit above bit 3 of a bf16 mantissa
-//         without reaching the exponent, so the high nibbles are shifted down)
-template <int FMT>
-__device__ __forceinline__ void expand_word(uint32_t w, uint32_t mask_lo, uint32_t mask_hi, uint32_t magic,
-                                            uint32_t& e02, uint32_t& e13, uint32_t& o02, uint32_t& o13) {
-  if (FMT == 0) {
-    const uint32_t w8 = w >> 8;
-    uint32_t a = (w & mask_lo) | magic, b = (w8 & mask_lo) | magic;
-    uint32_t c = (w & mask_hi) | magic, d = (w8 & mask_hi) | magic;
-    const __half2 k1024 = __half2half2(__float2half_rn(1024.f));
-    const __half2 k16th = __half2half2(__float2half_rn(0.0625f)), k64 = __half2half2(__float2half_rn(-64.f));
-    __half2 ra = __hsub2(*reinterpret_cast<__half2*>(&a), k1024), rb = __hsub2(*reinterpret_cast<__half2*>(&b), k1024);
-    __half2 rc = __hfma2(*reinterpret_cast<__half2*>(&c), k16th, k64), rd = __hfma2(*reinterpret_cast<__half2*>(&d), k16th, k64);
-    e02 = *reinterpret_cast<uint32_t*>(&ra); e13 = *reinterpret_cast<uint32_t*>(&rb);
-    o02 = *reinterpret_cast<uint32_t*>(&rc); o13 = *reinterpret_cast<uint32_t*>(&rd);
-  } else {
-    uint32_t a = (w & mask_lo) | magic, b = ((w >> 8) & mask_lo) | magic;
-    uint32_t c = ((w >> 4) & mask_lo) | magic, d = ((w >> 12) & mask_lo) | magic;
-    const __nv_bfloat162 k128 = __float2bfloat162_rn(128.f);
-    __nv_bfloat162 ra = __hsub2(*reinterpret_cast<__nv_bfloat162*>(&a), k128);
-    __nv_bfloat162 rb = __hsub2(*reinterpret_cast<__nv_bfloat162*>(&b), k128);
-    __nv_bfloat162 rc = __hsub2(*reinterpret_cast<__nv_bfloat162*>(&c), k128);
-    __nv_bfloat162 rd = __hsub2(*reinterpret_cast<__nv_bfloat162*>(&d), k128);
-    e02 = *reinterpret_cast<uint32_t*>(&ra); e13 = *reinterpret_cast<uint32_t*>(&rb);
-    o02 = *reinterpret_cast<uint32_t*>(&rc); o13 = *reinterpret_cast<uint32_t*>(&rd);
-  }
-}
-
 // Who issues inside a converged role warp: the MMA warp elects (that is what makes the issue cheap, see
 // elect_one); the TMA producers use a fixed lane - with an elected one, single CTAs produced wrong sums
 // now and then (1-3 of 250 CTAs per launch at 32000 x 5120), for a reason that was not found.
@@ -155,7 +75,6 @@ w4_umma_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   const int x_plane_bytes = p.NT * 128;
-  const int nt0 = min(p.NT, 256), nt1 = p.NT - nt0;      // tokens of the first / second accumulator
   const int x_stage_bytes = x_plane_bytes * p.planes;
   uint8_t* raw_ring = smem;
   const int RAW_ST = p.raw_stages, A_ST = p.a_stages;
@@ -245,8 +164,6 @@ w4_umma_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__
         if (U_LEADER_PROD) {
           mbar_expect_tx(&x_full[xs], (uint32_t)x_stage_bytes);
           tma_load_2d(x_ring + xs * x_stage_bytes, &xmap0, (int)(stage * U_STAGE_K), (int)m0, &x_full[xs]);
-          if (nt1 > 0)     // second box of 256 token rows (one plane only at this size)
-            tma_load_2d(x_ring + xs * x_stage_bytes + 256 * 128, &xmap0, (int)(stage * U_STAGE_K), (int)m0 + 256, &x_full[xs]);
           if (p.planes > 1)
             tma_load_2d(x_ring + xs * x_stage_bytes + x_plane_bytes, &xmap1, (int)(stage * U_STAGE_K), (int)m0, &x_full[xs]);
           UTRACE(1, i);
@@ -265,8 +182,7 @@ w4_umma_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__
   } else if (warp == 1) {
     // ===================== MMA issuer =====================
     {
-      const uint32_t idesc = make_idesc_f16(p.fmt, /*a M-major*/ 1, /*b K-major*/ 0, U_COLS, nt0);
-      const uint32_t idesc1 = make_idesc_f16(p.fmt, 1, 0, U_COLS, nt1 > 0 ? nt1 : 16);
+      const uint32_t idesc = make_idesc_f16(p.fmt, /*a M-major*/ 1, /*b K-major*/ 0, U_COLS, p.NT);
       // Descriptors are a constant plus (start address / 16) in the low bits: one addition per MMA.
       const uint64_t desc_a0 = make_desc_sw128(0, 8192, 1024), desc_b0 = make_desc_sw128(0, 16, 1024);
       const uint32_t a_ring16 = smem_u32(a_ring) >> 4, x_ring16 = smem_u32(x_ring) >> 4;
@@ -289,7 +205,6 @@ w4_umma_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__
           const uint64_t db = desc_b0 + (x16 + (uint32_t)(k16 * 32 >> 4));
           mma_f16_ss(tmem_acc, da, db, idesc, (i > 0 || k16 > 0) ? 1u : 0u);
           if (p.planes > 1) mma_f16_ss(tmem_acc, da, db + x_plane16, idesc, 1u);
-          if (nt1 > 0) mma_f16_ss(tmem_acc + 256, da, db + (uint32_t)(256 * 128 >> 4), idesc1, (i > 0 || k16 > 0) ? 1u : 0u);
         }
         UTRACE(7, i);
         mma_commit(&a_empty[as]);
@@ -456,12 +371,9 @@ UmmaPlan plan_w4_umma(int64_t M, int64_t N, int64_t K, int x_dtype) {
   const int64_t max_nt = pl.planes == 2 ? 128 : 256;
   const int64_t per_tile = std::min<int64_t>(M, max_nt);
   pl.NT = (int)(cdiv(per_tile, 16) * 16);
-  // above 256 tokens a CTA takes 512 (two 128 x 256 accumulators = all of TMEM): every expanded stage
-  // then feeds twice the tensor work, and the expansion is what bounds the kernel at large M
-  if (pl.planes == 1 && M > 256) pl.NT = 512;
   pl.mtiles = (int)cdiv(M, pl.NT);
   pl.ncg = (int)cdiv(N, U_COLS);
-  pl.tmem_cols = pl.NT <= 32 ? 32 : pl.NT <= 64 ? 64 : pl.NT <= 128 ? 128 : pl.NT <= 256 ? 256 : 512;
+  pl.tmem_cols = pl.NT <= 32 ? 32 : pl.NT <= 64 ? 64 : pl.NT <= 128 ? 128 : 256;
   const size_t x_stage = (size_t)pl.NT * 128 * pl.planes;
   // ring depths (<= 224 KB in all): raw and expanded-A rings hold one stage per active expansion warp
   // (8, or 4 when the activation tiles are large and the tensor pipe is the bound anyway)
@@ -561,7 +473,7 @@ int launch_w4_umma(const UmmaPlan& pl, const void* x, int x_dtype, const uint8_t
   CUtensorMap wmap, x0, x1;
   int rc = encode_tmap_2d_u8(&wmap, packed, (uint64_t)N, (uint64_t)(K / 2), (uint64_t)N, U_COLS, 32, 0);
   if (rc) return rc;
-  const uint32_t box_rows = (uint32_t)std::min(pl.NT, 256);
+  const uint32_t box_rows = (uint32_t)pl.NT;
   rc = encode_tmap_2d_b16(&x0, plane0, (uint64_t)K, (uint64_t)M, (uint64_t)K * 2, 64, box_rows);
   if (rc) return rc;
   rc = encode_tmap_2d_b16(&x1, plane1, (uint64_t)K, (uint64_t)M, (uint64_t)K * 2, 64, box_rows);

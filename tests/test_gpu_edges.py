@@ -213,3 +213,26 @@ def test_matmul_outside_and_inside_autograd(gg):
     traced = torch.jit.trace(lambda t: quantized_matmul(t, qm), (x,), check_trace=False)
     other = torch.randn_like(x)
     assert torch.equal(traced(other), quantized_matmul(other, qm))
+
+
+@pytest.mark.parametrize('M,K,N', [(33, 64, 256), (1, 136, 16), (20, 4104, 400), (256, 520, 272), (257, 1032, 528), (300, 128, 272),
+                                   (513, 4104, 400), (700, 3080, 1040), (1025, 72, 2064)])
+@pytest.mark.parametrize('dtype', [torch.float16, torch.bfloat16, torch.float32])
+@pytest.mark.parametrize('transpose', [False, True])
+def test_matmul_many_rows_edges_of_tiles(gg, M, K, N, dtype, transpose):
+    """Tiles of 256 weight rows by 256 or 512 tokens that are not full, contractions that end inside a stage, both
+    directions.  Against the dequantized product in fp64: the output's rounding, or for fp32 the planes' 2^-17 and
+    fp32 sums."""
+    from jax_gptq_b200 import quantized_matmul, QuantizedMatrix
+    g = torch.Generator(device='cuda').manual_seed(M + K + N)
+    packed = torch.randint(0, 256, (K // 2, N), generator=g, device='cuda', dtype=torch.uint8)
+    scale = 0.001 + 0.019 * torch.rand(N, generator=g, device='cuda')
+    zero = torch.randint(0, 16, (N,), generator=g, device='cuda').float()
+    x = torch.randn((M, N if transpose else K), generator=g, device='cuda').to(dtype)
+    dense = (torch.stack([packed & 15, packed >> 4], 1).reshape(K, N).double() - zero.double()) * scale.double()
+    want = x.double() @ (dense.T if transpose else dense)
+    qm = QuantizedMatrix(packed, zero, scale)
+    got = quantized_matmul(x, qm, transpose_b=transpose)
+    bound = {torch.float16: 2.0 ** -11, torch.bfloat16: 2.0 ** -8, torch.float32: 2e-5}[dtype]
+    assert ((got.double() - want).norm() / want.norm()).item() <= bound
+    assert torch.equal(got, quantized_matmul(x, qm, transpose_b=transpose))
