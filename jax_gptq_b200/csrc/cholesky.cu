@@ -10,14 +10,13 @@
 //   step k:  (1) factor diagonal block, invert it            (1 CTA)
 //            (2) panel below it  A[i,k] <- A[i,k] * inv_k^T   (row tiles)
 //            (3) X[k, <k]  <- -inv_k * S[k, <k]               (column tiles)
-//   trailing (4) A[i,j] -= A[i,k] A[j,k]^T                    (FFMA GEMM, lower tiles)
-//            (5) S[i>k, <=k] += A[i,k] X[k, <=k]              (FFMA GEMM)
+//   trailing (4) A[i,j] -= A[i,k] A[j,k]^T                    (lower tiles)
+//            (5) S[i>k, <=k] += A[i,k] X[k, <=k]
 //
 // (4) and (5) run once per outer block of four panels, with depth 256; inside an outer block
 // (2) and (3) apply the block's earlier panels to their tiles themselves.  S lives in the
 // not-yet-final part of X.  Everything is fp32 with IEEE division and square root.
 #include "common.cuh"
-#include "sgemm.cuh"
 #include <algorithm>
 #include <cstdlib>
 #include <cstring>
@@ -385,9 +384,10 @@ __device__ __forceinline__ void tile_mul_nn(float (&acc)[4][4], const float (*U)
 //   column block c < kb:  X[kb, c] <- -inv (S[kb, c] + sum_p A[kb, p] X[p, c])
 // The sums run before the wait for the diagonal kernel.  The CTA of a row block inside the outer block
 // (i < obe) then brings its diagonal block up to date with the tile it holds, A[i, i] -= A[i, kb] A[i, kb]^T,
-// so that the next diagonal kernel finds a finished block.
+// so that the next diagonal kernel finds a finished block.  With `mirror` the panel tile is also written transposed above
+// the diagonal (A[kb, i], which nothing else uses): the large trailing update reads it there.
 __global__ void __launch_bounds__(256)
-chol_tiles_kernel(float* __restrict__ A, float* __restrict__ X, int K, int kb, int ob, int obe, int tiles_below, int vec) {
+chol_tiles_kernel(float* __restrict__ A, float* __restrict__ X, int K, int kb, int ob, int obe, int tiles_below, int vec, int mirror) {
   __shared__ __align__(16) float U[CB][CS];
   __shared__ __align__(16) float V[CB][CS];
   const int r0 = kb * CB;
@@ -466,19 +466,295 @@ chol_tiles_kernel(float* __restrict__ A, float* __restrict__ X, int K, int kb, i
 #pragma unroll
     for (int j = 0; j < 4; ++j)
       if (i0 + ty + 16 * i < K && tx + 16 * j < nb) A[(int64_t)(i0 + ty + 16 * i) * K + r0 + tx + 16 * j] = acc[i][j];
-  if (ib >= obe) return;
+  const bool diag_next = ib < obe;
+  if (!diag_next && !mirror) return;
   __syncthreads();
 #pragma unroll
   for (int i = 0; i < 4; ++i)
 #pragma unroll
     for (int j = 0; j < 4; ++j) { U[ty + 16 * i][tx + 16 * j] = acc[i][j]; acc[i][j] = 0.f; }
   __syncthreads();
+  if (mirror && !diag_next) {
+    // rows of the outer block's own panels are never read transposed
+    const int r = tid & 63;
+    for (int c = tid >> 6; c < nb; c += 4)
+      if (i0 + r < K) A[(int64_t)(r0 + c) * K + i0 + r] = U[r][c];
+    return;
+  }
   tile_mul_nt(acc, U, U);
 #pragma unroll
   for (int i = 0; i < 4; ++i)
 #pragma unroll
     for (int j = 0; j < 4; ++j)
       if (i0 + ty + 16 * i < K && i0 + tx + 16 * j < K) A[(int64_t)(i0 + ty + 16 * i) * K + i0 + tx + 16 * j] -= acc[i][j];
+}
+
+__device__ __forceinline__ void cp_async16(float* dst, const float* src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
+}
+
+// ---- trailing updates of an outer block, both in one launch -------------------------------------------
+//   problem 0:  A[r, c] -= sum_k P[r, k] P[c, k]     lower tiles         problem 1:  S[r, c] += sum_k P[r, k] X[k, c]
+// with P the block's panel below it (depth 256).  Plain FP32 multiply-adds, one chain per element in increasing k, then
+// one addition: what a tile computes does not depend on its size.  Bound by the FP32 pipe when there are tiles for all
+// SMs (128 x 128, 8 x 8 per thread, packed pairs of multiply-adds), by a tile's own latency when there are not (64 x 64,
+// 4 x 4).  Stages of 32 in two buffers, 16-byte asynchronous copies, nothing transposed on the way.  An update at K = 4096
+// takes 84 us on average (128 x 128 x 8 tiles staged through registers: 104; this loop on k-contiguous rows: 134); the
+// stage as a whole 315 -> 277 us at K = 768, 2917 -> 2518 at K = 4096.
+struct UpdateParams {
+  const float* P; const float* PT; const float* X; float* A; float* S;     // PT: P transposed, rows of stride K as well
+  int K, depth, rows, cols0, cols1;      // rows of both; columns of problem 0 (= rows) and 1
+  int tiles0, tn1, vec;
+};
+
+constexpr int UBK = 32, UKS = UBK + 4;   // stage depth, row stride of a k-contiguous tile
+
+// tile (tm, tn) of the list: problem 0's lower tiles row by row, then problem 1's
+__device__ __forceinline__ bool update_tile(const UpdateParams& p, int& tm, int& tn) {
+  int t = blockIdx.x;
+  if (t >= p.tiles0) {
+    t -= p.tiles0;
+    tm = t / p.tn1; tn = t % p.tn1;
+    return true;
+  }
+  tm = (int)((sqrtf(8.f * (float)t + 1.f) - 1.f) * 0.5f);
+  while ((tm + 1) * (tm + 2) / 2 <= t) ++tm;
+  while (tm * (tm + 1) / 2 > t) --tm;
+  tn = t - tm * (tm + 1) / 2;
+  return false;
+}
+
+// Two multiply-adds, each rounded like fmaf.
+__device__ __forceinline__ void fma2(uint64_t& d, uint64_t a, uint64_t b) {
+  asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(d) : "l"(a), "l"(b));
+}
+__device__ __forceinline__ uint64_t twice(float a) {
+  uint64_t r;
+  asm("mov.b64 %0, {%1, %1};" : "=l"(r) : "f"(a));
+  return r;
+}
+
+// 128 x 128 tiles; both operands lie with their free index contiguous (the mirrored panel, X).  Needs p.vec and full stages.
+constexpr int ULS = 128;
+__global__ void __launch_bounds__(256, 2)
+chol_update_large_kernel(const UpdateParams p) {
+  extern __shared__ __align__(16) float usm[];                 // [2][A: UBK x 128, B: UBK x 128]
+  const int tid = threadIdx.x, ty = tid >> 4, tx = tid & 15;
+  int tm, tn;
+  const bool second = update_tile(p, tm, tn);
+  const int m0 = tm * 128, n0 = tn * 128, K = p.K;
+  const int ncol = second ? p.cols1 : p.cols0;
+  const float* Bp = second ? p.X : p.PT;
+  auto stage = [&](int kk, int buf) {
+    float* As = usm + buf * 2 * UBK * ULS;
+    float* Bs = As + UBK * ULS;
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const int k = (tid >> 5) + 8 * u, c = 4 * (tid & 31);
+      if (m0 + c < p.rows) cp_async16(As + k * ULS + c, p.PT + (int64_t)(kk + k) * K + m0 + c);
+      else *reinterpret_cast<float4*>(As + k * ULS + c) = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (n0 + c < ncol) cp_async16(Bs + k * ULS + c, Bp + (int64_t)(kk + k) * K + n0 + c);
+      else *reinterpret_cast<float4*>(Bs + k * ULS + c) = make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  uint64_t acc[8][4];
+#pragma unroll
+  for (int i = 0; i < 8; ++i)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) acc[i][j] = 0;
+  stage(0, 0);
+  for (int kk = 0, buf = 0; kk < p.depth; kk += UBK, buf ^= 1) {
+    if (kk + UBK < p.depth) { stage(kk + UBK, buf ^ 1); asm volatile("cp.async.wait_group 1;" ::: "memory"); }
+    else asm volatile("cp.async.wait_group 0;" ::: "memory");
+    __syncthreads();
+    const float* As = usm + buf * 2 * UBK * ULS + 4 * ty;
+    const float* Bs = usm + buf * 2 * UBK * ULS + UBK * ULS + 4 * tx;
+#pragma unroll 4
+    for (int k = 0; k < UBK; ++k) {
+      const float4 a0 = *reinterpret_cast<const float4*>(As + k * ULS), a1 = *reinterpret_cast<const float4*>(As + k * ULS + 64);
+      const ulonglong2 b0 = *reinterpret_cast<const ulonglong2*>(Bs + k * ULS), b1 = *reinterpret_cast<const ulonglong2*>(Bs + k * ULS + 64);
+      const float a[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        const uint64_t aa = twice(a[i]);
+        fma2(acc[i][0], aa, b0.x); fma2(acc[i][1], aa, b0.y);
+        fma2(acc[i][2], aa, b1.x); fma2(acc[i][3], aa, b1.y);
+      }
+    }
+    __syncthreads();
+  }
+  float* C = second ? p.S : p.A;
+  const float sign = second ? 1.f : -1.f;
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    const int r = m0 + (i < 4 ? 4 * ty + i : 64 + 4 * ty + i - 4);
+    if (r >= p.rows) continue;
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const int c = n0 + 64 * h + 4 * tx;
+      if (c < ncol) {                                       // ncol % 4 == 0
+        float4* dst = reinterpret_cast<float4*>(C + (int64_t)r * K + c);
+        const float2 v0 = *reinterpret_cast<const float2*>(&acc[i][2 * h]), v1 = *reinterpret_cast<const float2*>(&acc[i][2 * h + 1]);
+        float4 o = *dst;
+        o.x = fmaf(sign, v0.x, o.x); o.y = fmaf(sign, v0.y, o.y);
+        o.z = fmaf(sign, v1.x, o.z); o.w = fmaf(sign, v1.y, o.w);
+        *dst = o;
+      }
+    }
+  }
+}
+
+// 64 x 64 tiles for any K.
+__global__ void __launch_bounds__(256, 2)
+chol_update_kernel(const UpdateParams p) {
+  constexpr int B = 64, T = B / 16;                           // elements per thread and direction
+  constexpr int NS = B + 4;                                   // row stride of a tile with n contiguous
+  constexpr int STAGE = 2 * B * UKS;
+  static_assert(B * UKS >= UBK * NS, "either operand layout fits its half of a stage");
+  extern __shared__ __align__(16) float usm[];
+  const int tid = threadIdx.x, ty = tid >> 4, tx = tid & 15;
+  int tm, tn;
+  const bool second = update_tile(p, tm, tn);
+  const int m0 = tm * B, n0 = tn * B, K = p.K;
+  const int ncol = second ? p.cols1 : p.cols0;
+
+  auto stage = [&](int kk, int buf) {
+    float* As = usm + buf * STAGE;
+    float* Bs = As + B * UKS;
+    const int kn = min(UBK, p.depth - kk);
+    auto rows_kc = [&](float* dst, int r0, int rlim) {        // B rows of P, 32 k each
+      if (p.vec && kn == UBK) {
+#pragma unroll
+        for (int u = 0; u < B / 32; ++u) {
+          const int r = (tid >> 3) + 32 * u, c = 4 * (tid & 7);
+          if (r0 + r < rlim) cp_async16(dst + r * UKS + c, p.P + (int64_t)(r0 + r) * K + kk + c);
+          else *reinterpret_cast<float4*>(dst + r * UKS + c) = make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+      } else {
+        for (int i = tid; i < B * UBK; i += 256) {
+          const int r = i / UBK, c = i % UBK;
+          dst[r * UKS + c] = (r0 + r < rlim && c < kn) ? p.P[(int64_t)(r0 + r) * K + kk + c] : 0.f;
+        }
+      }
+    };
+    rows_kc(As, m0, p.rows);
+    if (!second) {
+      rows_kc(Bs, n0, p.rows);
+    } else if (p.vec && kn == UBK) {
+#pragma unroll
+      for (int u = 0; u < B / 32; ++u) {
+        const int i = tid + 256 * u, r = i / (B / 4), c = 4 * (i % (B / 4));
+        if (n0 + c < ncol) cp_async16(Bs + r * NS + c, p.X + (int64_t)(kk + r) * K + n0 + c);
+        else *reinterpret_cast<float4*>(Bs + r * NS + c) = make_float4(0.f, 0.f, 0.f, 0.f);
+      }
+    } else {
+      for (int i = tid; i < UBK * B; i += 256) {
+        const int r = i / B, c = i % B;
+        Bs[r * NS + c] = (r < kn && n0 + c < ncol) ? p.X[(int64_t)(kk + r) * K + n0 + c] : 0.f;
+      }
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+
+  float acc[T][T];
+#pragma unroll
+  for (int i = 0; i < T; ++i)
+#pragma unroll
+    for (int j = 0; j < T; ++j) acc[i][j] = 0.f;
+  stage(0, 0);
+  for (int kk = 0, buf = 0; kk < p.depth; kk += UBK, buf ^= 1) {
+    if (kk + UBK < p.depth) { stage(kk + UBK, buf ^ 1); asm volatile("cp.async.wait_group 1;" ::: "memory"); }
+    else asm volatile("cp.async.wait_group 0;" ::: "memory");
+    __syncthreads();
+    const float* As = usm + buf * STAGE + ty * UKS;
+    const float* Bs = usm + buf * STAGE + B * UKS;
+    if (!second) {
+#pragma unroll 2
+      for (int k = 0; k < UBK; k += 4) {
+        float4 u[T];
+#pragma unroll
+        for (int i = 0; i < T; ++i) u[i] = *reinterpret_cast<const float4*>(As + 16 * i * UKS + k);
+#pragma unroll
+        for (int j = 0; j < T; ++j) {
+          const float4 w = *reinterpret_cast<const float4*>(Bs + (tx + 16 * j) * UKS + k);
+#pragma unroll
+          for (int i = 0; i < T; ++i) {
+            acc[i][j] = fmaf(u[i].x, w.x, acc[i][j]); acc[i][j] = fmaf(u[i].y, w.y, acc[i][j]);
+            acc[i][j] = fmaf(u[i].z, w.z, acc[i][j]); acc[i][j] = fmaf(u[i].w, w.w, acc[i][j]);
+          }
+        }
+      }
+    } else {
+#pragma unroll 2
+      for (int k = 0; k < UBK; k += 4) {
+        float4 u[T];
+#pragma unroll
+        for (int i = 0; i < T; ++i) u[i] = *reinterpret_cast<const float4*>(As + 16 * i * UKS + k);
+#pragma unroll
+        for (int k1 = 0; k1 < 4; ++k1)
+#pragma unroll
+          for (int j4 = 0; j4 < T / 4; ++j4) {
+            const float4 w = *reinterpret_cast<const float4*>(Bs + (k + k1) * NS + 64 * j4 + 4 * tx);
+#pragma unroll
+            for (int i = 0; i < T; ++i) {
+              const float a = k1 == 0 ? u[i].x : k1 == 1 ? u[i].y : k1 == 2 ? u[i].z : u[i].w;
+              acc[i][4 * j4] = fmaf(a, w.x, acc[i][4 * j4]); acc[i][4 * j4 + 1] = fmaf(a, w.y, acc[i][4 * j4 + 1]);
+              acc[i][4 * j4 + 2] = fmaf(a, w.z, acc[i][4 * j4 + 2]); acc[i][4 * j4 + 3] = fmaf(a, w.w, acc[i][4 * j4 + 3]);
+            }
+          }
+      }
+    }
+    __syncthreads();
+  }
+
+  float* C = second ? p.S : p.A;
+#pragma unroll
+  for (int i = 0; i < T; ++i) {
+    const int r = m0 + ty + 16 * i;
+    if (r >= p.rows) continue;
+    float* row = C + (int64_t)r * K;
+    if (!second) {
+#pragma unroll
+      for (int j = 0; j < T; ++j) {
+        const int c = n0 + tx + 16 * j;
+        if (c < ncol) row[c] -= acc[i][j];
+      }
+    } else {
+#pragma unroll
+      for (int j4 = 0; j4 < T / 4; ++j4) {
+        const int c = n0 + 64 * j4 + 4 * tx;
+        if (p.vec && c + 3 < ncol) {
+          float4 o = *reinterpret_cast<const float4*>(row + c);
+          o.x += acc[i][4 * j4]; o.y += acc[i][4 * j4 + 1]; o.z += acc[i][4 * j4 + 2]; o.w += acc[i][4 * j4 + 3];
+          *reinterpret_cast<float4*>(row + c) = o;
+        } else {
+#pragma unroll
+          for (int j = 0; j < 4; ++j)
+            if (c + j < ncol) row[c + j] += acc[i][4 * j4 + j];
+        }
+      }
+    }
+  }
+}
+
+template <auto Kern>
+static int launch_update_tiles(UpdateParams p, int B, int smem, cudaStream_t s) {
+  prefer_shared_carveout<Kern>();
+  struct AttrTag {};
+  once_per_device<AttrTag>([&]() { return (int)cudaFuncSetAttribute(reinterpret_cast<const void*>(Kern), cudaFuncAttributeMaxDynamicSharedMemorySize, smem); });
+  const int tr = (int)cdiv(p.rows, B);
+  p.tiles0 = tr * (tr + 1) / 2;
+  p.tn1 = (int)cdiv(p.cols1, B);
+  Kern<<<(unsigned)(p.tiles0 + tr * p.tn1), 256, smem, s>>>(p);
+  return check_launch("chol_update");
+}
+
+// Large tiles from one per SM on (they compute twice as much per byte from shared memory); fewer leave SMs idle
+// while the small ones do not.
+static bool large_update(int K, int c_end, int depth, int vec) {
+  const int64_t tr = cdiv(K - c_end, 128);
+  return vec && depth % UBK == 0 && tr * (tr + 1) / 2 + tr * cdiv(c_end, 128) >= (int64_t)sm_count();
 }
 
 // ---- final: L[i][j] = X[K-1-j][K-1-i] (i >= j), 0 above the diagonal -----------
@@ -565,6 +841,7 @@ extern "C" int jgq_damp_invert(float* W, int64_t N, float* H, int64_t K, float d
   for (int ob = 0; ob < nblk; ob += COB) {
     const int c_begin = ob * CB;                                   // first column of the outer block
     const int c_end = std::min(Ki, (ob + COB) * CB);               // one past its last column
+    const bool large = c_end < Ki && large_update(Ki, c_end, c_end - c_begin, vec);
     for (int kb = ob; kb < std::min(nblk, ob + COB); ++kb) {
       const int r1 = std::min(Ki, (kb + 1) * CB);      // first row below the diagonal block
       const int below = Ki - r1;
@@ -585,7 +862,7 @@ extern "C" int jgq_damp_invert(float* W, int64_t N, float* H, int64_t K, float d
       if (e == cudaSuccess && tiles_below + kb > 0) {
         cfg.gridDim = dim3((unsigned)(tiles_below + kb));
         cfg.numAttrs = 1;
-        e = cudaLaunchKernelEx(&cfg, chol_tiles_kernel, A, X, Ki, kb, ob, std::min(nblk, ob + COB), tiles_below, vec);
+        e = cudaLaunchKernelEx(&cfg, chol_tiles_kernel, A, X, Ki, kb, ob, std::min(nblk, ob + COB), tiles_below, vec, large ? 1 : 0);
         note_launches(1);
       }
       if (e != cudaSuccess) { cudaGetLastError(); return fail(JGQ_ERR_CUDA, "damp_invert: %s", cudaGetErrorString(e)); }
@@ -594,12 +871,16 @@ extern "C" int jgq_damp_invert(float* W, int64_t N, float* H, int64_t K, float d
       // the block's whole panel Pb = A[c_end:, c_begin:c_end] at once:
       // A[c_end:, c_end:] -= Pb Pb^T (lower tiles)   and   S[c_end:, :c_end] += Pb X[c_begin:c_end, :c_end]
       const int below = Ki - c_end, depth = c_end - c_begin;
-      const float* Pb = A + (int64_t)c_end * K + c_begin;
-      GemmParams g0 = make_gemm_params(Pb, K, Pb, K, A + (int64_t)c_end * K + c_end, K, below, below, depth,
-                                       -1.f, 1.f, 1);
-      GemmParams g1 = make_gemm_params(Pb, K, X + (int64_t)c_begin * K, K, X + (int64_t)c_end * K, K,
-                                       below, c_end, depth, 1.f, 1.f, 0);
-      const int rc = launch_sgemm_dual(g0, true, g1, false, s);
+      UpdateParams up;
+      memset(&up, 0, sizeof(up));
+      up.P = A + (int64_t)c_end * K + c_begin;
+      up.X = X + (int64_t)c_begin * K;
+      up.A = A + (int64_t)c_end * K + c_end;
+      up.S = X + (int64_t)c_end * K;
+      up.K = Ki; up.depth = depth; up.rows = below; up.cols0 = below; up.cols1 = c_end; up.vec = vec;
+      up.PT = A + (int64_t)c_begin * K + c_end;
+      const int rc = large ? launch_update_tiles<chol_update_large_kernel>(up, 128, 4 * UBK * ULS * (int)sizeof(float), s)
+                           : launch_update_tiles<chol_update_kernel>(up, 64, 4 * 64 * UKS * (int)sizeof(float), s);
       if (rc) return rc;
     }
   }

@@ -66,6 +66,20 @@ __device__ __forceinline__ float divide_exact(float a, float b, float y) {
   return fmaf(e, y, q);
 }
 
+// Products with near-fp32 accuracy on the tensor cores: every operand is split as x = hi + lo with hi = tf32(x), lo =
+// tf32(x - hi), and accumulated as lo*hi + hi*lo + hi*hi.  The split keeps 22 of the 24 significand bits, so it is for
+// updates that tolerate 2^-21 relative error per product (the lazy-batch update), not for the Cholesky sweep.
+__device__ __forceinline__ void split_tf32(float x, uint32_t& hi, uint32_t& lo) {
+  asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(hi) : "f"(x));
+  const float r = x - __uint_as_float(hi);
+  asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(lo) : "f"(r));
+}
+__device__ __forceinline__ void mma_tf32(float (&d)[4], const uint32_t (&a)[4], const uint32_t (&b)[2]) {
+  asm volatile("mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
+               : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+               : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]));
+}
+
 // split_tf32 in integer arithmetic (the conversion unit is a quarter as wide): rounding half away from zero is an
 // addition to the magnitude's bits.  For finite values.
 __device__ __forceinline__ void split_tf32_alu(float x, uint32_t& hi, uint32_t& lo) {
@@ -540,7 +554,7 @@ static int run_quantize(float* W, const float* L, const float* scale, const floa
     if (e != cudaSuccess) { cudaGetLastError(); return fail(JGQ_ERR_CUDA, "gptq_block: %s", cudaGetErrorString(e)); }
     if (!fused && rest > 0) {
       const int rc = launch_sgemm(true, false, L + (int64_t)(start + bs) * K + start, K, W + (int64_t)start * N, N,
-                                  W + (int64_t)(start + bs) * N, N, rest, (int)N, bs, -1.f, 1.f, 0, s, 1, 0, 0);
+                                  W + (int64_t)(start + bs) * N, N, rest, (int)N, bs, -1.f, 1.f, 0, s);
       if (rc) return rc;
     }
   }
