@@ -16,7 +16,7 @@
 // rounded multiply and subtract, which is exactly the sequence of roundings the reference's unrolled loop performs,
 // so a block is bit-identical to the fp32 oracle given the same inputs.  The lazy-batch update is three TF32
 // products per term on the tensor cores (mma.sync, increasing contraction index).
-// Measured per 128-row block: alone (N = 32) 84 -> 26 us; with its share of the update, K = N = 4096, 46 + 77 -> 78 us.
+// Measured per 128-row block: alone (N = 32) 84 -> 26 us; with its share of the update, K = N = 4096, 46 + 77 -> 64 us.
 // The loop's code is kept short on purpose (groups of four steps, rolled loops): with the steps of a sub-block unrolled,
 // three of ten issue slots of the kernel went to instruction fetches and a block took 33 us.
 #include "common.cuh"
@@ -105,7 +105,9 @@ __device__ __forceinline__ void cp_async16(uint32_t dst, const void* src) {
 
 // W[m0 .. + 127 behind the block, n0 .. + 63] -= L[rows, previous block] @ errors of the previous block, three TF32
 // products per term.  A rank-128 update is bound by its traffic (96 KB of operands and 64 KB of W read and written per
-// tile): two 32-deep stages in flight, two CTAs per SM.
+// tile): two 32-deep stages in flight, two CTAs per SM.  Without any arithmetic the tiles of a K = N = 4096 loop take 0.96 of
+// 1.6 ms; the rest is the operands' split and the products' latency, hence one split per operand ahead of three runs of
+// eight independent products (the whole loop 2.18 -> 2.05 ms against split and products term by term).
 __device__ __forceinline__ void tail_tile(const QuantParams& p, float* smem, int tile) {
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, q = lane & 3;
   const int m0 = (tile / p.tail_tn) * TBM, n0 = (tile % p.tail_tn) * TBN;
@@ -161,7 +163,7 @@ __device__ __forceinline__ void tail_tile(const QuantParams& p, float* smem, int
     asm volatile("bar.sync 6, 256;" ::: "memory");
     const float* As = smem + buf * TSTAGE_FLOATS + wm * TAS;
     const float* Bs = smem + buf * TSTAGE_FLOATS + TBM * TAS + wn;
-#pragma unroll 1
+#pragma unroll 2
     for (int k8 = 0; k8 < TBK && kk + k8 < bs; k8 += 8) {
       uint32_t ah[2][4], al[2][4];
 #pragma unroll
@@ -172,19 +174,26 @@ __device__ __forceinline__ void tail_tile(const QuantParams& p, float* smem, int
         split_tf32_alu(ap[4], ah[i][2], al[i][2]);
         split_tf32_alu(ap[8 * TAS + 4], ah[i][3], al[i][3]);
       }
+      uint32_t bh[4][2], bl[4][2];
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
         const float* bp = Bs + (k8 + q) * TBS + 8 * j + g;
-        uint32_t bh[2], bl[2];
-        split_tf32(bp[0], bh[0], bl[0]);
-        split_tf32(bp[4 * TBS], bh[1], bl[1]);
-#pragma unroll
-        for (int i = 0; i < 2; ++i) mma_tf32(acc[i][j], al[i], bh);
-#pragma unroll
-        for (int i = 0; i < 2; ++i) mma_tf32(acc[i][j], ah[i], bl);
-#pragma unroll
-        for (int i = 0; i < 2; ++i) mma_tf32(acc[i][j], ah[i], bh);
+        split_tf32_alu(bp[0], bh[j][0], bl[j][0]);
+        split_tf32_alu(bp[4 * TBS], bh[j][1], bl[j][1]);
       }
+      // eight independent accumulators between two products of one
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+#pragma unroll
+        for (int i = 0; i < 2; ++i) mma_tf32(acc[i][j], al[i], bh[j]);
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+#pragma unroll
+        for (int i = 0; i < 2; ++i) mma_tf32(acc[i][j], ah[i], bl[j]);
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+#pragma unroll
+        for (int i = 0; i < 2; ++i) mma_tf32(acc[i][j], ah[i], bh[j]);
     }
     asm volatile("bar.sync 6, 256;" ::: "memory");
   }
@@ -319,7 +328,9 @@ gptq_block_kernel(const QuantParams p) {
       const float cv = c[i * QCH + lane];
       reinterpret_cast<QT*>(p.Q)[o] = from_f32<QT>(__fmul_rn(sc, __fsub_rn(cv, zr)));
       if (p.codes) p.codes[o] = (uint8_t)cv;
-      p.W[o] = e[i * QES + lane];
+      // Not finite: stored as the NaN that survives the operand split of the tail tiles (an infinity's low part would be one)
+      const float err = e[i * QES + lane];
+      p.W[o] = fabsf(err) <= 3.402823466e38f ? err : __uint_as_float(0x7fc00000u);
     }
   };
   // The helpers' half-warps take two neighbouring rows, two channels per lane: a broadcast of L then feeds two
