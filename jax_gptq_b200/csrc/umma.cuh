@@ -64,6 +64,18 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volati
   }
 }
 
+// For waits that last as long as a whole tile: sleeps between polls, so that the warps that are working keep the
+// issue slots.
+__device__ __forceinline__ bool mbar_wait_long(uint64_t* bar, uint32_t parity, volatile int* abort) {
+  const long long t0 = clock64();
+  while (!mbar_try_wait(bar, parity)) {
+    if (*abort) return false;
+    if (clock64() - t0 > kWaitBudgetCycles) { *abort = 1; return false; }
+    __nanosleep(256);
+  }
+  return true;
+}
+
 // ---- TMA --------------------------------------------------------------------
 __device__ __forceinline__ void tma_load_2d(void* smem_dst, const CUtensorMap* map, int c0, int c1, uint64_t* bar) {
   asm volatile(

@@ -312,7 +312,7 @@ static size_t w4_forward_need(int64_t M, int64_t N, int64_t K, int x_dtype) {
 // the GPU time of 9 row counts from 33 to 2048 on seven weight shapes from 768 x 2304 to 8192 x 28672:
 //   single CTA   13 per wave, 0.3 to 0.7 per stage (more with the tile's tokens), 9 per slice of a split contraction and 128
 //                tokens for the slices' exchange;
-//   pair         7 per wave of 74, 0.45 per stage with one block of 256 tokens, 0.7 with two.
+//   pair         see plan_w4_pair.
 // The single-CTA kernel keeps few rows on long contractions (64 rows, K = 11008, N = 4096: 76 against 82 us; 128 rows of
 // fp32: 87 against 133); more than 256 rows of 16-bit activations always go to the pairs (2048 rows, 4096 x 11008: 293
 // against 176 us).  The transposed product takes the pairs whenever they can run (33 rows, 4096 x 4096: 108 against
@@ -326,11 +326,10 @@ static PairPlan w4_pair_choice(int64_t M, int64_t N, int64_t K, int x_dtype, int
   const UmmaPlan up = plan_w4_umma(M, N, K, x_dtype);
   if (!up.use) return pp;
   const int sms = sm_count();
-  const double pair = (double)cdiv(pp.units, std::max(1, sms / 2)) * ((pp.planes == 2 ? 0.7 : 0.45) * (double)cdiv(pp.depth, 64) + 7.0);
   const double stage = up.planes == 2 ? 0.35 + 0.0022 * up.NT : 0.3 + 0.0016 * up.NT;
   const double single = (double)cdiv((int64_t)up.ncg * up.mtiles * up.ksplit, sms) * (stage * up.stages_per_split + 13.0) +
                         (up.ksplit > 1 ? 9.0 / 128.0 * up.NT * up.ksplit : 0.0);
-  pp.use = pair + 8.0 < 0.93 * (single + 10.0);
+  pp.use = pp.us < 0.93 * (single + 10.0);
   return pp;
 }
 

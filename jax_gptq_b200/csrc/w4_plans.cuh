@@ -35,8 +35,10 @@ int launch_w4_tb(const void* x, int x_dtype, const uint8_t* packed, const void* 
 
 // CTA-pair kernel for many tokens, forward and transposed (w4_pair.cu); use: it can run (the dispatcher chooses)
 struct PairPlan {
-  int use; int planes; int tile; int rows; int depth; int nrp; int units; int64_t Np;
+  int use; int planes; int rows; int depth; int nrp; int nt; int items; int twos; int halves; int cols; int64_t Np;
   size_t plane_bytes; size_t ws_bytes;
+  int G;                            // pairs
+  double us;                        // estimate
 };
 PairPlan plan_w4_pair(int64_t M, int64_t N, int64_t K, int x_dtype, int transpose_b);
 int launch_w4_pair(const PairPlan& pl, const void* x, int x_dtype, const uint8_t* packed, const void* zero, const void* scale,

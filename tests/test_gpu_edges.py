@@ -236,3 +236,29 @@ def test_matmul_many_rows_edges_of_tiles(gg, M, K, N, dtype, transpose):
     bound = {torch.float16: 2.0 ** -11, torch.bfloat16: 2.0 ** -8, torch.float32: 2e-5}[dtype]
     assert ((got.double() - want).norm() / want.norm()).item() <= bound
     assert torch.equal(got, quantized_matmul(x, qm, transpose_b=transpose))
+
+
+@pytest.mark.parametrize('M,K,N', [(65, 256, 4096), (97, 136, 272), (150, 72, 640), (200, 512, 4800), (512, 136, 8208),
+                                   (768, 136, 8208), (1300, 200, 10256), (2300, 72, 10256)])
+@pytest.mark.parametrize('dtype', [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize('transpose', [False, True])
+def test_matmul_many_rows_blocks_and_rounds(gg, M, K, N, dtype, transpose):
+    """Blocks of fewer than 256 tokens, and work lists of several items per pair of SMs (whole rounds, halved
+    items, a last odd column), in both directions: the weights' sides are exchanged for the transposed product.
+    Against the dequantized product in fp64, the whole and each element."""
+    from jax_gptq_b200 import quantized_matmul, QuantizedMatrix
+    if transpose:
+        K, N = N, K // 16 * 16
+    g = torch.Generator(device='cuda').manual_seed(M + K + N)
+    packed = torch.randint(0, 256, (K // 2, N), generator=g, device='cuda', dtype=torch.uint8)
+    scale = 0.001 + 0.019 * torch.rand(N, generator=g, device='cuda')
+    zero = torch.randint(0, 16, (N,), generator=g, device='cuda').float()
+    x = torch.randn((M, N if transpose else K), generator=g, device='cuda').to(dtype)
+    dense = (torch.stack([packed & 15, packed >> 4], 1).reshape(K, N).double() - zero.double()) * scale.double()
+    want = x.double() @ (dense.T if transpose else dense)
+    got = quantized_matmul(x, QuantizedMatrix(packed, zero, scale), transpose_b=transpose)
+    bound = {torch.bfloat16: 2.0 ** -8, torch.float32: 2e-5}[dtype]
+    assert ((got.double() - want).norm() / want.norm()).item() <= bound
+    # no element is missing or misplaced: 16 x the bound, of the element and its row together (a missing stage or tile is of order one)
+    row = want.norm(dim=1, keepdim=True) / want.shape[1] ** 0.5
+    assert ((got.double() - want).abs() / (row + want.abs())).max().item() <= 16 * bound
