@@ -19,11 +19,13 @@
 //     code * 2^-24 (code * 2^-20 for the high nibble, where it sits four bits up), which the tensor
 //     core multiplies exactly.  So an operand register costs 1.5 integer instructions;
 //   * the activations are brought into that operand order once per stage and warp (shared memory,
-//     a few hundred bytes): pairs (x[2j], x[2j+2]) and (x[2j+1], x[2j+3]) / 16, the 1/16 making up
-//     for the high nibbles' position.  Activations below 2^-10 in magnitude lose bits beyond 2^-24
-//     there (absolute), far below the f16 output's resolution;
+//     a few hundred bytes): pairs (x[2j], x[2j+2]) and (x[2j+1], x[2j+3]), as they are.  An f16 MMA takes
+//     the low nibbles of two steps, another their high nibbles into an accumulator of its own, which counts
+//     a sixteenth: no activation is scaled, so none is rounded however small it is.  What an MMA reads of the
+//     two steps lies side by side (even-index pairs of both, then in a second half the odd-index pairs), so that
+//     one 8-byte load fills a register pair: with the pairs of a step side by side the moves cost up to 9 %;
 //   * sum_k x[k], which the zero point multiplies, comes from one more MMA per step whose weight
-//     operand is the constant (1, 1, 16, 16).
+//     operand is all ones.
 // out[m, n] = scale[n] * (2^24 * acc[m, n] - zero[n] * sum_k x[m, k]).
 //
 // bf16 activations: a bf16 subnormal times an activation would leave fp32's range, so the codes get an exponent
@@ -32,7 +34,7 @@
 // (x = hi + lo + O(2^-17 |x|)), two MMAs on the same expanded weights.
 // More than eight token rows are groups of eight on the same expanded weights.
 // Measured (GPU time per call, back to back): bf16 8 x 4096 x 11008 20.1 -> 18.0 us against the streaming kernel; f16 32 x 768 x
-// 2304 28.5 -> 11.8 us against two passes of it.
+// 2304 28.5 -> 12.3 us against two passes of it.
 //
 // Launch overlap: the kernel is launched with programmatic stream serialization.  It sets up its
 // barriers and, when the caller declared the weights settled (JGQ_W4_WEIGHTS_SETTLED), issues its
@@ -82,6 +84,9 @@ __device__ __forceinline__ uint2 lds64(uint32_t addr) {
   asm volatile("ld.shared.v2.u32 {%0, %1}, [%2];" : "=r"(v.x), "=r"(v.y) : "r"(addr));
   return v;
 }
+__device__ __forceinline__ void sts32(uint32_t addr, uint32_t a) {
+  asm volatile("st.shared.u32 [%0], %1;" ::"r"(addr), "r"(a) : "memory");
+}
 __device__ __forceinline__ void sts64(uint32_t addr, uint32_t a, uint32_t b) {
   asm volatile("st.shared.v2.u32 [%0], {%1, %2};" ::"r"(addr), "r"(a), "r"(b) : "memory");
 }
@@ -103,18 +108,22 @@ __device__ __forceinline__ void mma_bf16(float (&d)[4], uint32_t a0, uint32_t a1
 template <typename XT> struct GemvType;
 template <> struct GemvType<__half> {
   static constexpr int PLANES = 1;
+  static constexpr int ACCS = 2;                                       // low and high nibbles apart
   static constexpr float UP = 16777216.f;                              // 2^24: the codes enter as code * 2^-24
-  static constexpr uint32_t ONES_LO = 0x3C003C00u, ONES_HI = 0x4C004C00u;   // (1, 1) and (16, 16)
+  static constexpr uint32_t ONES = 0x3C003C00u;
   // four operand registers (low / high nibbles of two channels) of the two byte rows' permuted bytes
   __device__ static __forceinline__ void expand(uint32_t p0, uint32_t p1, uint32_t (&a)[4]) {
     a[0] = p0 & 0x000F000Fu; a[1] = p1 & 0x000F000Fu; a[2] = p0 & 0x00F000F0u; a[3] = p1 & 0x00F000F0u;
   }
-  __device__ static __forceinline__ void mma(float (&d)[4], const uint32_t (&a)[4], uint2 b) { mma_f16(d, a[0], a[1], a[2], a[3], b.x, b.y); }
+  __device__ static __forceinline__ void mma(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+    mma_f16(d, a0, a1, a2, a3, b0, b1);
+  }
 };
 template <> struct GemvType<__nv_bfloat16> {
   static constexpr int PLANES = 1;
+  static constexpr int ACCS = 1;
   static constexpr float UP = 1.f;
-  static constexpr uint32_t ONES_LO = 0x3F803F80u, ONES_HI = 0x3F803F80u;
+  static constexpr uint32_t ONES = 0x3F803F80u;
   __device__ static __forceinline__ uint32_t code(uint32_t v) {
     uint32_t r = (v & 0x000F000Fu) | 0x43004300u;
     const __nv_bfloat162 h = __hsub2(*reinterpret_cast<__nv_bfloat162*>(&r), __float2bfloat162_rn(128.f));
@@ -123,7 +132,9 @@ template <> struct GemvType<__nv_bfloat16> {
   __device__ static __forceinline__ void expand(uint32_t p0, uint32_t p1, uint32_t (&a)[4]) {
     a[0] = code(p0); a[1] = code(p1); a[2] = code(p0 >> 4); a[3] = code(p1 >> 4);
   }
-  __device__ static __forceinline__ void mma(float (&d)[4], const uint32_t (&a)[4], uint2 b) { mma_bf16(d, a[0], a[1], a[2], a[3], b.x, b.y); }
+  __device__ static __forceinline__ void mma(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+    mma_bf16(d, a0, a1, a2, a3, b0, b1);
+  }
 };
 template <> struct GemvType<float> : GemvType<__nv_bfloat16> { static constexpr int PLANES = 2; };
 
@@ -143,6 +154,7 @@ w4_gemv_kernel(const __grid_constant__ CUtensorMap wmap, const GemvParams p) {
   constexpr int STEPS = ROWS / 8;                  // 8 byte rows (16 contraction indices) per MMA step
   constexpr int PAIRS = ROWS / 2;                  // 8-byte operand pairs per token row and stage
   constexpr int XROW = PAIRS * 8 + 32;             // bytes per staged token row (+32: rows land on different banks)
+  constexpr int XROW_ODD = PAIRS * 4;              // ACCS == 2: the odd-index pairs of a row
   constexpr int XWARP = NT * PL * XROW;            // planes one after the other
   extern __shared__ uint8_t smem_raw[];
   uint8_t* ring = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -193,12 +205,17 @@ w4_gemv_kernel(const __grid_constant__ CUtensorMap wmap, const GemvParams p) {
     for (int j = 0; j < GV_NST && j < nstage; ++j) issue_stage(j);
 
   constexpr int NG = (NT + 7) / 8;               // groups of eight token rows
-  float acc[NG][2][4], accx[NG][4];
+  constexpr int ACCS = T::ACCS;
+  float acc[NG][2][ACCS][4], accx[NG][4];
   auto clear_acc = [&]() {
 #pragma unroll
     for (int q = 0; q < NG; ++q)
 #pragma unroll
-      for (int i = 0; i < 4; ++i) { acc[q][0][i] = 0.f; acc[q][1][i] = 0.f; accx[q][i] = 0.f; }
+      for (int i = 0; i < 4; ++i) {
+        accx[q][i] = 0.f;
+#pragma unroll
+        for (int h = 0; h < ACCS; ++h) { acc[q][0][h][i] = 0.f; acc[q][1][h][i] = 0.f; }
+      }
   };
   clear_acc();
 
@@ -216,7 +233,7 @@ w4_gemv_kernel(const __grid_constant__ CUtensorMap wmap, const GemvParams p) {
   const uint32_t chunk = 2 * warp + (g >> 2), inchunk = 4 * (g & 3);
   const uint32_t off0 = (2 * t) * WCOLS + ((chunk ^ (2 * t)) << 4) + inchunk;
   const uint32_t off1 = (2 * t + 1) * WCOLS + ((chunk ^ (2 * t + 1)) << 4) + inchunk;
-  const uint32_t ones[4] = {T::ONES_LO, T::ONES_LO, T::ONES_HI, T::ONES_HI};
+  constexpr uint32_t ones = T::ONES;
 
   int gid = g_begin, st = st_begin;
   bool alive = true;
@@ -262,34 +279,49 @@ w4_gemv_kernel(const __grid_constant__ CUtensorMap wmap, const GemvParams p) {
           sts64(dst + NT * XROW, lo[0], lo[1]);
         } else {
           const uint32_t ev = __byte_perm(xv[r][h].x, xv[r][h].y, 0x5410);
-          uint32_t od = __byte_perm(xv[r][h].x, xv[r][h].y, 0x7632);
-          if constexpr (std::is_same<XT, __half>::value) {
-            const __half2 o2 = __hmul2(*reinterpret_cast<__half2*>(&od), __float2half2_rn(0.0625f));      // the high nibbles sit four bits up
-            od = *reinterpret_cast<const uint32_t*>(&o2);
+          const uint32_t od = __byte_perm(xv[r][h].x, xv[r][h].y, 0x7632);
+          if constexpr (ACCS == 2) {
+            // pair `lane & 3` of step lane / 4: 8 bytes per pair for two steps
+            const uint32_t dst2 = xs_warp + r * XROW + h * 128 + (lane >> 3) * 32 + (lane & 3) * 8 + ((lane >> 2) & 1) * 4;
+            sts32(dst2, ev);
+            sts32(dst2 + XROW_ODD, od);
+          } else {
+            sts64(dst, ev, od);
           }
-          sts64(dst, ev, od);
         }
       }
     __syncwarp();
     if (alive) {
       const uint32_t tile = ring_u32 + slot * STAGE_BYTES;
 #pragma unroll
-      for (int sl = 0; sl < STEPS; ++sl) {
-        const uint32_t w1 = lds32(tile + sl * (8 * WCOLS) + off0);
-        const uint32_t w2 = lds32(tile + sl * (8 * WCOLS) + off1);
-        const uint32_t p0 = __byte_perm(w1, w2, 0x4400), p1 = __byte_perm(w1, w2, 0x5511);
-        const uint32_t p2 = __byte_perm(w1, w2, 0x6622), p3 = __byte_perm(w1, w2, 0x7733);
-        uint32_t a0[4], a1[4];
-        T::expand(p0, p1, a0);
-        T::expand(p2, p3, a1);
+      for (int sl = 0; sl < STEPS; sl += ACCS) {
+        uint32_t a0[ACCS][4], a1[ACCS][4];         // per step: low nibbles, then high nibbles, of the two channel tiles
+#pragma unroll
+        for (int h = 0; h < ACCS; ++h) {
+          const uint32_t w1 = lds32(tile + (sl + h) * (8 * WCOLS) + off0);
+          const uint32_t w2 = lds32(tile + (sl + h) * (8 * WCOLS) + off1);
+          T::expand(__byte_perm(w1, w2, 0x4400), __byte_perm(w1, w2, 0x5511), a0[h]);
+          T::expand(__byte_perm(w1, w2, 0x6622), __byte_perm(w1, w2, 0x7733), a1[h]);
+        }
 #pragma unroll
         for (int q = 0; q < NG; ++q)
 #pragma unroll
           for (int pl = 0; pl < PL; ++pl) {
-            const uint2 xb = lds64(xs_read[q] + pl * (q * 8 + g < p.M ? NT * XROW : 0) + sl * 32);
-            T::mma(acc[q][0], a0, xb);
-            T::mma(acc[q][1], a1, xb);
-            T::mma(accx[q], ones, xb);
+            const uint32_t xr = xs_read[q] + pl * (q * 8 + g < p.M ? NT * XROW : 0) + sl * (32 / ACCS);
+            const uint2 xb = lds64(xr);
+            if constexpr (ACCS == 2) {
+              const uint2 xc = lds64(xr + XROW_ODD);
+              T::mma(acc[q][0][0], a0[0][0], a0[0][1], a0[1][0], a0[1][1], xb.x, xb.y);
+              T::mma(acc[q][1][0], a1[0][0], a1[0][1], a1[1][0], a1[1][1], xb.x, xb.y);
+              T::mma(accx[q], ones, ones, ones, ones, xb.x, xb.y);
+              T::mma(acc[q][0][1], a0[0][2], a0[0][3], a0[1][2], a0[1][3], xc.x, xc.y);
+              T::mma(acc[q][1][1], a1[0][2], a1[0][3], a1[1][2], a1[1][3], xc.x, xc.y);
+              T::mma(accx[q], ones, ones, ones, ones, xc.x, xc.y);
+            } else {
+              T::mma(acc[q][0][0], a0[0][0], a0[0][1], a0[0][2], a0[0][3], xb.x, xb.y);
+              T::mma(acc[q][1][0], a1[0][0], a1[0][1], a1[0][2], a1[0][3], xb.x, xb.y);
+              T::mma(accx[q], ones, ones, ones, ones, xb.x, xb.y);
+            }
           }
       }
       __syncwarp();
@@ -326,7 +358,11 @@ w4_gemv_kernel(const __grid_constant__ CUtensorMap wmap, const GemvParams p) {
     for (int q = 0; q < NG; ++q)
 #pragma unroll
       for (int e = 0; e < 2; ++e) {
-        v[q][e] = make_float4(acc[q][0][e] + poison, acc[q][0][2 + e] + poison, acc[q][1][e] + poison, acc[q][1][2 + e] + poison);
+        auto sum = [&](int tile, int i) {
+          if constexpr (ACCS == 2) return fmaf(acc[q][tile][1][i], 0.0625f, acc[q][tile][0][i]) + poison;
+          else return acc[q][tile][0][i] + poison;
+        };
+        v[q][e] = make_float4(sum(0, e), sum(0, 2 + e), sum(1, e), sum(1, 2 + e));
         xsum[q][e] = accx[q][e];
       }
     bool write_out = true;

@@ -262,3 +262,21 @@ def test_matmul_many_rows_blocks_and_rounds(gg, M, K, N, dtype, transpose):
     # no element is missing or misplaced: 16 x the bound, of the element and its row together (a missing stage or tile is of order one)
     row = want.norm(dim=1, keepdim=True) / want.shape[1] ** 0.5
     assert ((got.double() - want).abs() / (row + want.abs())).max().item() <= 16 * bound
+
+
+@pytest.mark.parametrize('M', [1, 2, 8, 16, 17, 24, 32, 33, 64])
+@pytest.mark.parametrize('K,N', [(768, 2304), (136, 48), (270, 37)])
+def test_matmul_small_f16_activations(gg, M, K, N):
+    """f16 activations far below one, rows of different magnitudes: every one enters the product as it is, so all that is
+    lost is the output's rounding, 2^-11 of the value or half a step of the subnormals (2^-25), row by row."""
+    from jax_gptq_b200 import quantized_matmul, QuantizedMatrix
+    g = torch.Generator(device='cuda').manual_seed(M + K)
+    packed = torch.randint(0, 256, (K // 2, N), generator=g, device='cuda', dtype=torch.uint8)
+    scale = 0.001 + 0.019 * torch.rand(N, generator=g, device='cuda')
+    zero = torch.randint(0, 16, (N,), generator=g, device='cuda').float()
+    dense = (torch.stack([packed & 15, packed >> 4], 1).reshape(K, N).double() - zero.double()) * scale.double()
+    for s in (1e-3, 1e-4, 1e-5):
+        x = (torch.randn((M, K), generator=g, device='cuda') * s * 2.0 ** -(torch.arange(M, device='cuda') % 3)[:, None]).half()
+        want = x.double() @ dense
+        err = (quantized_matmul(x, QuantizedMatrix(packed, zero, scale)).double() - want).norm(dim=1)
+        assert torch.all(err <= 2.0 ** -11 * want.norm(dim=1) + 2.0 ** -25 * N ** 0.5)
