@@ -194,6 +194,114 @@ static __global__ void split_x_bf16_kernel(const float* __restrict__ X, __nv_bfl
   }
 }
 
+// Four consecutive values as fp32: one load where `vec`, else what lies below `lim`, zeros behind.
+template <typename T>
+__device__ __forceinline__ void load4(float (&f)[4], const T* p, uint32_t n, uint32_t lim, bool vec) {
+  __align__(16) T e[4];
+  if (vec) {
+    using V = typename std::conditional<sizeof(T) == 4, float4, uint2>::type;
+    *reinterpret_cast<V*>(e) = *reinterpret_cast<const V*>(p + n);
+  } else {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) e[i] = n + i < lim ? p[n + i] : from_f32<T>(0.f);
+  }
+#pragma unroll
+  for (int i = 0; i < 4; ++i) f[i] = to_f32<T>(e[i]);
+}
+
+// The activations of the transposed product: xs = x * scale times a power of two of the token row, as two f16 planes hi + lo
+// [M][Np] (zero beyond N), and c[m] = (sum_n x scale zero, the inverse power of two).  PAIRED: channels 0, 2, 1, 3 within each four.
+// The power of two brings the largest product of the row to [2^13, 2^14).  The planes then hold 22 bits of every element
+// down to 2^-16 of it, whatever the row's magnitude (gradients of a mean over many tokens are far below f16's range).
+// One CTA per row, which keeps 4 J THREADS products in registers between the two uses and forms what is longer twice.
+template <typename XT, typename ZST, int THREADS, int J, bool PAIRED>
+__global__ void __launch_bounds__(THREADS, 2048 / THREADS)
+tb_prep_kernel(const XT* __restrict__ x, const ZST* __restrict__ scale, const ZST* __restrict__ zero,
+               uint32_t N, uint32_t Np, __half* __restrict__ hi, __half* __restrict__ lo, float2* __restrict__ c, int vec) {
+  const int64_t m = blockIdx.x;
+  __shared__ float pmax[THREADS / 32], psum[THREADS / 32];
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  x += m * N;
+  hi += m * Np;
+  lo += m * Np;
+  float v[J][4], big = 0.f, s = 0.f;
+  auto products = [&](float (&p)[4], uint32_t n) {
+    float a[4], z[4];
+    load4<XT>(p, x, n, N, vec != 0);
+    load4<ZST>(a, scale, n, N, vec != 0);
+    load4<ZST>(z, zero, n, N, vec != 0);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      p[i] = n + i < N ? __fmul_rn(p[i], a[i]) : 0.f;
+      big = fmaxf(big, fabsf(p[i]));
+      s = fmaf(p[i], z[i], s);
+    }
+  };
+#pragma unroll
+  for (int j = 0; j < J; ++j) {
+    const uint32_t n = 4 * (threadIdx.x + THREADS * j);
+    if (n < N) products(v[j], n);
+  }
+  for (uint32_t n = 4 * (threadIdx.x + THREADS * J); n < N; n += 4 * THREADS) {
+    float p[4];
+    products(p, n);
+  }
+  // fixed-order reductions: lanes by shuffle, warps in index order
+  for (int o = 16; o > 0; o >>= 1) {
+    big = fmaxf(big, __shfl_xor_sync(0xffffffffu, big, o));
+    s += __shfl_xor_sync(0xffffffffu, s, o);
+  }
+  if ((threadIdx.x & 31) == 0) { pmax[threadIdx.x >> 5] = big; psum[threadIdx.x >> 5] = s; }
+  __syncthreads();
+  for (int w = 0; w < THREADS / 32; ++w) big = fmaxf(big, pmax[w]);
+  const uint32_t e = min(max(__float_as_uint(big) >> 23, 14u), 254u);      // biased exponent; rows below 2^-113 get 2^126
+  const float up = __uint_as_float((267u - e) << 23);
+  if (threadIdx.x == 0) {
+    float t = 0.f;
+    for (int w = 0; w < THREADS / 32; ++w) t += psum[w];
+    c[m] = make_float2(t, __uint_as_float((e - 13u) << 23));
+  }
+  auto store = [&](const float (&p)[4], uint32_t n) {
+    __half h[4], l[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const float q = p[PAIRED && (i == 1 || i == 2) ? 3 - i : i] * up;
+      h[i] = __float2half_rn(q);
+      l[i] = __float2half_rn(q - __half2float(h[i]));
+    }
+    *reinterpret_cast<uint2*>(hi + n) = *reinterpret_cast<const uint2*>(h);
+    *reinterpret_cast<uint2*>(lo + n) = *reinterpret_cast<const uint2*>(l);
+  };
+  const float none[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+  for (int j = 0; j < J; ++j) {
+    const uint32_t n = 4 * (threadIdx.x + THREADS * j);
+    if (n < N) store(v[j], n);
+    else if (n < Np) store(none, n);
+  }
+  for (uint32_t n = 4 * (threadIdx.x + THREADS * J); n < Np; n += 4 * THREADS) {
+    float p[4] = {0.f, 0.f, 0.f, 0.f};
+    if (n < N) products(p, n);
+    store(p, n);
+  }
+}
+
+// Blocks as wide as a row needs with few products per thread: 32 registers, so that an SM's 2048 threads hide the loads, which
+// is what bounds it (2048 rows of 768 channels with 32 products per thread and half the threads: 4 us more).  Wide ones also
+// for few rows, where one row's latency counts (one row of 32000 channels with 256 threads: 12 us more).
+template <typename XT, typename ZST, bool PAIRED>
+static int launch_tb_prep(const XT* x, const void* scale, const void* zero, int64_t rows, int64_t N, int64_t Np, __half* hi,
+                          __half* lo, float2* c, cudaStream_t s) {
+  const int vec = N % 4 == 0 && aligned(x, 4 * sizeof(XT)) && aligned(scale, 4 * sizeof(ZST)) && aligned(zero, 4 * sizeof(ZST));
+  auto go = [&](auto kern, int threads) {
+    kern<<<(unsigned)rows, threads, 0, s>>>(x, (const ZST*)scale, (const ZST*)zero, (uint32_t)N, (uint32_t)Np, hi, lo, c, vec);
+    return check_launch("w4_matmul_tb_prep");
+  };
+  if (N <= 1024) return go(tb_prep_kernel<XT, ZST, 256, 1, PAIRED>, 256);
+  if (N > 4096 || rows <= sm_count()) return go(tb_prep_kernel<XT, ZST, 1024, 2, PAIRED>, 1024);
+  return N <= 2048 ? go(tb_prep_kernel<XT, ZST, 256, 2, PAIRED>, 256) : go(tb_prep_kernel<XT, ZST, 512, 2, PAIRED>, 512);
+}
+
 // 8 codes of one 32-bit word (4 channels x {k even, k odd}) -> four 2-channel registers.
 // e02 / e13: k even, channels (0,2) / (1,3);  o02 / o13: k odd.
 // The integer / logic pipe is the scarce one (half rate), so the constants come from kernel

@@ -388,13 +388,13 @@ extern "C" int jgq_w4_matmul(const void* x, int x_dtype, const uint8_t* packed,
   if (M == 0) return JGQ_OK;
   cudaStream_t s = (cudaStream_t)stream;
   if (transpose_b) {
-    const size_t need_tb = w4_tb_workspace_bytes(M, N);
+    const size_t need_tb = w4_tb_min_workspace_bytes(M, N);
     JGQ_REQUIRE(ws && ws_bytes >= need_tb, JGQ_ERR_WORKSPACE, "w4_matmul: workspace %zu < %zu bytes", ws_bytes, need_tb);
     JGQ_REQUIRE(aligned(ws, 256), JGQ_ERR_ALIGN, "w4_matmul: workspace must be 256-byte aligned");
     const PairPlan pp = w4_pair_choice(M, N, K, x_dtype, 1);
     if (pp.use && pp.ws_bytes <= ws_bytes && aligned(packed, 16))
       return launch_w4_pair(pp, x, x_dtype, packed, zero, scale, zs_dtype, out, M, N, K, 1, ws, s);
-    return launch_w4_tb(x, x_dtype, packed, zero, scale, zs_dtype, out, M, N, K, ws, s);
+    return launch_w4_tb(x, x_dtype, packed, zero, scale, zs_dtype, out, M, N, K, ws, ws_bytes, s);
   }
   JGQ_REQUIRE(aligned(x, 8), JGQ_ERR_ALIGN, "w4_matmul: x must be 8-byte aligned");
   const size_t need = w4_forward_need(M, N, K, x_dtype);

@@ -2,6 +2,7 @@
 //
 //   forward     out[m, n] = scale[n] * ( sum_k x[m, k] code[k, n]  -  zero[n] * sum_k x[m, k] )
 //   transposed  out[m, k] = sum_n xs[m, n] code[k, n]  -  c[m],   xs = x * scale,  c[m] = sum_n xs[m, n] zero[n]
+//               (xs times a power of two of its row, see tb_prep_kernel, which the epilogue takes off again)
 //
 // The weights are the MMA's 256 rows (output channels n, or contraction-side outputs k in the transposed product),
 // the tokens its columns.  A CTA of the pair expands the nibbles of its own 128 rows and loads its half of the
@@ -68,7 +69,7 @@ constexpr int P_TMEM_COLS = 512;
 
 struct PairParams {
   const void* zero; const void* scale; void* out;
-  const float* tok;            // [M]: sum_k x[m, k] (forward) or c[m] (transposed)
+  const float* tok;            // forward: [M] sum_k x[m, k]; transposed: [M][2] c[m] and the power of two for the sums
   int64_t M, N, K;
   int rows, depth;             // weight rows (N or K) and contraction length (K or N)
   int planes, nrp;             // activation planes, row pairs (256 weight rows each)
@@ -352,7 +353,15 @@ w4_pair_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__
         tc_fence_after();
         const int ntok = (int)min((int64_t)256, p.M - m0);
         for (int c = final_item ? 32 * share : 0; c < ntok; c += final_item ? 96 : 32) {
-          const float tok = c + lane < ntok ? __ldg(p.tok + m0 + c + lane) : 0.f;
+          // one value per token comes by shuffle, a pair through the 16 bytes that every token's row of the buffer has left
+          float tok = 0.f;
+          if (TB) {
+            if (c + lane < ntok)
+              *reinterpret_cast<float2*>(buf + lane * P_OUT_STRIDE + 128) = *reinterpret_cast<const float2*>(p.tok + 2 * (int64_t)(m0 + c + lane));
+            __syncwarp();
+          } else if (c + lane < ntok) {
+            tok = p.tok[m0 + c + lane];
+          }
           uint32_t v[32];
           if (done) {
             tmem_ld_32x32(tmem_acc + (uint32_t)(256 * b) + ((uint32_t)(32 * q) << 16) + (uint32_t)c, v);
@@ -362,9 +371,16 @@ w4_pair_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__
             for (int i = 0; i < 32; ++i) v[i] = 0x7fc00000u;
           }
 #pragma unroll
-          for (int i = 0; i < 32; ++i)
-            *reinterpret_cast<XT*>(buf + i * P_OUT_STRIDE + lrow * (int)sizeof(XT)) =
-                from_f32<XT>(sc * (__uint_as_float(v[i]) - zr * __shfl_sync(0xffffffffu, tok, i)));
+          for (int i = 0; i < 32; ++i) {
+            float o;
+            if (TB) {
+              const float2 t = *reinterpret_cast<const float2*>(buf + i * P_OUT_STRIDE + 128);
+              o = fmaf(__uint_as_float(v[i]), t.y, -t.x);
+            } else {
+              o = sc * (__uint_as_float(v[i]) - zr * __shfl_sync(0xffffffffu, tok, i));
+            }
+            *reinterpret_cast<XT*>(buf + i * P_OUT_STRIDE + lrow * (int)sizeof(XT)) = from_f32<XT>(o);
+          }
           __syncwarp();
 #pragma unroll
           for (int i0 = 0; i0 < 32; i0 += TPW) {
@@ -400,42 +416,6 @@ w4_pair_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__
   }
 }
 
-// xs = x * scale as two f16 planes [M][Np] (zero beyond N), channels 0, 2, 1, 3 within each four, and
-// c[m] = sum_n xs[m, n] zero[n].  One CTA per token row, four channels per thread and step.
-template <typename XT, typename ZST>
-__global__ void __launch_bounds__(256)
-pair_tb_prep_kernel(const XT* __restrict__ x, const void* __restrict__ scale, const void* __restrict__ zero,
-                    int64_t N, int64_t Np, __half* __restrict__ hi, __half* __restrict__ lo, float* __restrict__ c) {
-  const int64_t m = blockIdx.x;
-  __shared__ float part[8];
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-  float s = 0.f;
-  for (int64_t n = 4 * (int64_t)threadIdx.x; n < Np; n += 1024) {
-    __half h[4], l[4];
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const int64_t ni = n + (i == 1 ? 2 : i == 2 ? 1 : i);
-      float v = 0.f;
-      if (ni < N) {
-        v = __fmul_rn(to_f32<XT>(x[m * N + ni]), zs_to_f32<ZST>(scale, ni));
-        s = fmaf(v, zs_to_f32<ZST>(zero, ni), s);
-      }
-      h[i] = __float2half_rn(v);
-      l[i] = __float2half_rn(v - __half2float(h[i]));
-    }
-    *reinterpret_cast<uint2*>(hi + m * Np + n) = *reinterpret_cast<const uint2*>(h);
-    *reinterpret_cast<uint2*>(lo + m * Np + n) = *reinterpret_cast<const uint2*>(l);
-  }
-  for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-  if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = s;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    float t = 0.f;
-    for (int w = 0; w < 8; ++w) t += part[w];
-    c[m] = t;
-  }
-}
-
 // ------------------------------------------------------------------ host ----
 PairPlan plan_w4_pair(int64_t M, int64_t N, int64_t K, int x_dtype, int transpose_b) {
   PairPlan pl;
@@ -463,7 +443,8 @@ PairPlan plan_w4_pair(int64_t M, int64_t N, int64_t K, int x_dtype, int transpos
   pl.us = (double)rounds * two + (double)cdiv(std::max<int64_t>(0, pl.halves + odd - room), pairs) * one + 12.0;
   pl.Np = cdiv(N, P_STAGE_K) * P_STAGE_K;
   pl.plane_bytes = pl.planes == 1 ? 0 : align_up((size_t)M * (transpose_b ? pl.Np : K) * 2, 256);
-  pl.ws_bytes = W4_TICKET_REGION + align_up((size_t)M * sizeof(float), 256) + 2 * pl.plane_bytes;
+  pl.tok_bytes = align_up((size_t)M * (transpose_b ? sizeof(float2) : sizeof(float)), 256);
+  pl.ws_bytes = W4_TICKET_REGION + pl.tok_bytes + 2 * pl.plane_bytes;
   pl.use = 1;
   return pl;
 }
@@ -502,14 +483,14 @@ template <typename XT, typename ZST>
 static int launch_pair_type(const PairPlan& pl, PairParams& p, const void* x, const uint8_t* packed, int transpose_b, uint8_t* ws, cudaStream_t s) {
   const int64_t M = p.M, N = p.N, K = p.K;
   float* tok = (float*)(ws + W4_TICKET_REGION);
-  uint8_t* planes = ws + W4_TICKET_REGION + align_up((size_t)M * sizeof(float), 256);
+  uint8_t* planes = ws + W4_TICKET_REGION + pl.tok_bytes;
   p.tok = tok;
   const void* plane[2] = {x, x};
   if (pl.planes == 2) { plane[0] = planes; plane[1] = planes + pl.plane_bytes; }
   int fmt;
   if (transpose_b) {
-    pair_tb_prep_kernel<XT, ZST><<<(unsigned)M, 256, 0, s>>>((const XT*)x, p.scale, p.zero, N, pl.Np, (__half*)plane[0], (__half*)plane[1], tok);
-    JGQ_LAUNCHED();
+    const int rc = launch_tb_prep<XT, ZST, true>((const XT*)x, p.scale, p.zero, M, N, pl.Np, (__half*)plane[0], (__half*)plane[1], (float2*)tok, s);
+    if (rc) return rc;
     fmt = 0;
   } else if (pl.planes == 2) {
     const int64_t total = M * K;

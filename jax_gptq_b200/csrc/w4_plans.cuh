@@ -30,13 +30,14 @@ int launch_w4_stream(const StreamPlan& pl, const void* x, int x_dtype, const uin
 
 // transposed product (w4_tb.cu)
 size_t w4_tb_workspace_bytes(int64_t M, int64_t N);
+size_t w4_tb_min_workspace_bytes(int64_t M, int64_t N);
 int launch_w4_tb(const void* x, int x_dtype, const uint8_t* packed, const void* zero, const void* scale, int zs_dtype,
-                 void* out, int64_t M, int64_t N, int64_t K, void* ws, cudaStream_t s);
+                 void* out, int64_t M, int64_t N, int64_t K, void* ws, size_t ws_bytes, cudaStream_t s);
 
 // CTA-pair kernel for many tokens, forward and transposed (w4_pair.cu); use: it can run (the dispatcher chooses)
 struct PairPlan {
   int use; int planes; int rows; int depth; int nrp; int nt; int items; int twos; int halves; int cols; int64_t Np;
-  size_t plane_bytes; size_t ws_bytes;
+  size_t plane_bytes; size_t tok_bytes; size_t ws_bytes;
   int G;                            // pairs
   double us;                        // estimate
 };

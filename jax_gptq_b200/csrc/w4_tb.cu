@@ -7,8 +7,8 @@
 //
 //   out[m, k] = sum_n xs[m, n] * code[k, n]  -  c[m],     xs = x * scale,   c[m] = sum_n xs[m, n] * zero[n]
 //
-// A small first kernel forms xs (fp32 product, then split into two f16 planes hi + lo so that fp32
-// activations keep 22 bits) and c.  The main kernel is a tensor-core GEMM whose 16-row MMA operand is the
+// A small first kernel forms xs (fp32 product, times a power of two of the row, see tb_prep_kernel, then split into two
+// f16 planes hi + lo so that fp32 activations keep 22 bits) and c.  The main kernel is a tensor-core GEMM whose 16-row MMA operand is the
 // packed weight matrix as it lies in memory: a byte row j holds codes k = 2j (low nibbles) and k = 2j + 1
 // (high nibbles) of consecutive channels, which is the contraction direction here.  One byte permute puts
 // two neighbouring channels' bytes into the two halves of a register; the and-mask 0x000F000F makes the
@@ -32,35 +32,6 @@ constexpr int TB_KOUT = 128;          // outputs k per CTA (64 byte rows)
 constexpr int TB_NS = 64;             // channels per contraction slice
 constexpr int TB_ROWB = 2 * TB_NS + 8;   // bytes per staged xs row (f16) with padding
 
-// xs planes [Mp][Np] (f16, zero padded), c[M]
-template <typename XT, typename ZST>
-__global__ void __launch_bounds__(256)
-tb_prep_kernel(const XT* __restrict__ x, const void* __restrict__ scale, const void* __restrict__ zero,
-               int64_t M, int64_t N, int64_t Np, __half* __restrict__ hi, __half* __restrict__ lo, float* __restrict__ c) {
-  const int64_t m = blockIdx.x;
-  __shared__ float part[8];
-  float s = 0.f;
-  for (int64_t n = threadIdx.x; n < Np; n += 256) {
-    float v = 0.f;
-    if (m < M && n < N) {
-      v = __fmul_rn(to_f32<XT>(x[m * N + n]), zs_to_f32<ZST>(scale, n));
-      s = fmaf(v, zs_to_f32<ZST>(zero, n), s);
-    }
-    const __half h = __float2half_rn(v);
-    hi[m * Np + n] = h;
-    lo[m * Np + n] = __float2half_rn(v - __half2float(h));
-  }
-  // fixed-order reduction: lanes by shuffle, warps in index order
-  for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-  if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = s;
-  __syncthreads();
-  if (threadIdx.x == 0 && m < M) {
-    float t = 0.f;
-    for (int w = 0; w < 8; ++w) t += part[w];
-    c[m] = t;
-  }
-}
-
 __device__ __forceinline__ void tb_mma(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
   asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
                : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
@@ -71,7 +42,7 @@ __device__ __forceinline__ void tb_mma(float (&d)[4], uint32_t a0, uint32_t a1, 
 template <typename XT>
 __global__ void __launch_bounds__(128)
 w4_tb_mma_kernel(const uint8_t* __restrict__ packed, const __half* __restrict__ hi, const __half* __restrict__ lo,
-                 const float* __restrict__ c, XT* __restrict__ out, int64_t M, int64_t N, int64_t K, int64_t Np) {
+                 const float2* __restrict__ c, XT* __restrict__ out, int64_t M, int64_t N, int64_t K, int64_t Np) {
   __shared__ __align__(16) uint8_t xs_s[2][2][TB_TOK * TB_ROWB];       // [buffer][plane][token row]
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int g = lane >> 2, t = lane & 3;
@@ -97,7 +68,8 @@ w4_tb_mma_kernel(const uint8_t* __restrict__ packed, const __half* __restrict__ 
       for (int i = 0; i < 4; ++i) {
         const int piece = threadIdx.x + 128 * i;
         const int row = piece >> 3, col = piece & 7;
-        const uint4 v = *reinterpret_cast<const uint4*>(src + (m0 + row) * Np + (int64_t)sl * TB_NS + 8 * col);
+        // rows past the end repeat the last one; their sums are not written
+        const uint4 v = *reinterpret_cast<const uint4*>(src + min(m0 + row, M - 1) * Np + (int64_t)sl * TB_NS + 8 * col);
         // the padded row stride is a multiple of 8 bytes, not of 16: two 8-byte stores
         *reinterpret_cast<uint2*>(&xs_s[buf][pl][row * TB_ROWB + 16 * col]) = make_uint2(v.x, v.y);
         *reinterpret_cast<uint2*>(&xs_s[buf][pl][row * TB_ROWB + 16 * col + 8]) = make_uint2(v.z, v.w);
@@ -174,9 +146,9 @@ w4_tb_mma_kernel(const uint8_t* __restrict__ packed, const __half* __restrict__ 
       for (int e = 0; e < 2; ++e) {
         const int64_t m = m0 + 8 * tg + 2 * t + e;
         if (m < M) {
-          const float cm = c[m];
-          out[m * K + 2 * j] = from_f32<XT>(acc[s][tg][e] * up_even - cm);
-          out[m * K + 2 * j + 1] = from_f32<XT>(acc[s][tg][2 + e] * up_odd - cm);
+          const float2 cm = c[m];
+          out[m * K + 2 * j] = from_f32<XT>(fmaf(acc[s][tg][e] * up_even, cm.y, -cm.x));
+          out[m * K + 2 * j + 1] = from_f32<XT>(fmaf(acc[s][tg][2 + e] * up_odd, cm.y, -cm.x));
         }
       }
   }
@@ -184,32 +156,45 @@ w4_tb_mma_kernel(const uint8_t* __restrict__ packed, const __half* __restrict__ 
 
 // The planes lie behind the ticket region that the forward kernels keep at the start of a shared workspace
 // (they expect to find it zero).
-size_t w4_tb_workspace_bytes(int64_t M, int64_t N) {
+static size_t tb_bytes(int64_t M, int64_t N) {            // for all rows in one pass
+  const int64_t Np = cdiv(N, TB_NS) * TB_NS;
+  return W4_TICKET_REGION + align_up((size_t)M * Np * 2, 256) * 2 + align_up((size_t)M * sizeof(float2), 256);
+}
+// What a call is refused without: whole tiles of token rows and four bytes a row.  That is less than tb_bytes when M
+// is (nearly) a multiple of the tile; the rows then take several passes.
+size_t w4_tb_min_workspace_bytes(int64_t M, int64_t N) {
   const int64_t Mp = cdiv(M, TB_TOK) * TB_TOK, Np = cdiv(N, TB_NS) * TB_NS;
   return W4_TICKET_REGION + align_up((size_t)Mp * Np * 2, 256) * 2 + align_up((size_t)M * sizeof(float), 256);
 }
+size_t w4_tb_workspace_bytes(int64_t M, int64_t N) { return std::max(tb_bytes(M, N), w4_tb_min_workspace_bytes(M, N)); }
 
 template <typename XT, typename ZST>
 static int launch_tb_inst(const void* x, const uint8_t* packed, const void* zero, const void* scale, void* out,
-                          int64_t M, int64_t N, int64_t K, void* ws, cudaStream_t s) {
-  const int64_t Mp = cdiv(M, TB_TOK) * TB_TOK, Np = cdiv(N, TB_NS) * TB_NS;
-  const size_t plane = align_up((size_t)Mp * Np * 2, 256);
+                          int64_t M, int64_t N, int64_t K, void* ws, size_t ws_bytes, cudaStream_t s) {
+  const int64_t Np = cdiv(N, TB_NS) * TB_NS;
+  int64_t step = M;                                       // token rows per pass
+  while (tb_bytes(step, N) > ws_bytes) step = (step + 1) / 2;
+  const size_t plane = align_up((size_t)step * Np * 2, 256);
   char* base = (char*)ws + W4_TICKET_REGION;
   __half* hi = (__half*)base;
   __half* lo = (__half*)(base + plane);
-  float* c = (float*)(base + 2 * plane);
-  tb_prep_kernel<XT, ZST><<<(unsigned)Mp, 256, 0, s>>>((const XT*)x, scale, zero, M, N, Np, hi, lo, c);
-  JGQ_LAUNCHED();
-  dim3 grid((unsigned)cdiv(K, TB_KOUT), (unsigned)(Mp / TB_TOK));
-  w4_tb_mma_kernel<XT><<<grid, 128, 0, s>>>(packed, hi, lo, c, (XT*)out, M, N, K, Np);
-  return check_launch("w4_matmul_tb");
+  float2* c = (float2*)(base + 2 * plane);
+  for (int64_t m = 0; m < M; m += step) {
+    const int64_t rows = std::min(step, M - m);
+    const int rc = launch_tb_prep<XT, ZST, false>((const XT*)x + m * N, scale, zero, rows, N, Np, hi, lo, c, s);
+    if (rc) return rc;
+    dim3 grid((unsigned)cdiv(K, TB_KOUT), (unsigned)cdiv(rows, TB_TOK));
+    w4_tb_mma_kernel<XT><<<grid, 128, 0, s>>>(packed, hi, lo, c, (XT*)out + m * K, rows, N, K, Np);
+    JGQ_LAUNCHED();
+  }
+  return JGQ_OK;
 }
 
 int launch_w4_tb(const void* x, int x_dtype, const uint8_t* packed, const void* zero, const void* scale, int zs_dtype,
-                 void* out, int64_t M, int64_t N, int64_t K, void* ws, cudaStream_t s) {
-#define JGQ_TB(XT)                                                                                          \
-  return zs_dtype == JGQ_F32 ? launch_tb_inst<XT, float>(x, packed, zero, scale, out, M, N, K, ws, s)       \
-                             : launch_tb_inst<XT, __half>(x, packed, zero, scale, out, M, N, K, ws, s)
+                 void* out, int64_t M, int64_t N, int64_t K, void* ws, size_t ws_bytes, cudaStream_t s) {
+#define JGQ_TB(XT)                                                                                                 \
+  return zs_dtype == JGQ_F32 ? launch_tb_inst<XT, float>(x, packed, zero, scale, out, M, N, K, ws, ws_bytes, s)    \
+                             : launch_tb_inst<XT, __half>(x, packed, zero, scale, out, M, N, K, ws, ws_bytes, s)
   if (x_dtype == JGQ_F32) { JGQ_TB(float); }
   if (x_dtype == JGQ_F16) { JGQ_TB(__half); }
   JGQ_TB(__nv_bfloat16);

@@ -280,3 +280,60 @@ def test_matmul_small_f16_activations(gg, M, K, N):
         want = x.double() @ dense
         err = (quantized_matmul(x, QuantizedMatrix(packed, zero, scale)).double() - want).norm(dim=1)
         assert torch.all(err <= 2.0 ** -11 * want.norm(dim=1) + 2.0 ** -25 * N ** 0.5)
+
+
+@pytest.mark.parametrize('M,K,N', [(1, 256, 1024), (137, 768, 1024), (300, 272, 4112), (1, 256, 909), (64, 768, 909), (137, 256, 909)])
+@pytest.mark.parametrize('dtype', [torch.float16, torch.bfloat16, torch.float32])
+def test_transposed_matmul_of_any_magnitude(gg, M, K, N, dtype):
+    """Gradients of a mean over many tokens are far below one, scaled losses far above: both kernels of the transposed
+    product, rows of different magnitudes and rows of zeros in one call.  Row by row against fp64: the output's rounding,
+    and the planes' 2^-22 with fp32 sums over up to 4112 channels, which are of the codes and of the zero points apart:
+    2e-5 of either one's norm, also where their difference is smaller."""
+    from jax_gptq_b200 import quantized_matmul, QuantizedMatrix
+    g = torch.Generator(device='cuda').manual_seed(M + K + N)
+    packed = torch.randint(0, 256, (K // 2, N), generator=g, device='cuda', dtype=torch.uint8)
+    scale = 0.001 + 0.019 * torch.rand(N, generator=g, device='cuda')
+    zero = torch.randint(0, 16, (N,), generator=g, device='cuda').float()
+    dense = (torch.stack([packed & 15, packed >> 4], 1).reshape(K, N).double() - zero.double()) * scale.double()
+    qm = QuantizedMatrix(packed, zero, scale)
+    offset = zero.double() * scale.double()
+    bound = {torch.float16: 2.0 ** -11, torch.bfloat16: 2.0 ** -8, torch.float32: 0.0}[dtype]
+    floor = 2.0 ** -25 * K ** 0.5 if dtype == torch.float16 else 0.0         # half a step of f16's subnormals
+    for s in (1.0, 1e-3, 1e-4) if dtype == torch.float16 else (1.0, 1e-3, 1e-4, 1e-5, 1e-6, 1e-8, 1e-30, 1e6, 1e20):
+        row = torch.tensor([1.0, 2.0 ** -6, 3.0, 0.0])[torch.arange(M) % 4].cuda()[:, None]
+        x = (torch.randn((M, N), generator=g, device='cuda') * s * row).to(dtype)
+        want = x.double() @ dense.T
+        got = quantized_matmul(x, qm, transpose_b=True)
+        parts = (want + (x.double() @ offset)[:, None]).norm(dim=1) + (x.double() @ offset).abs() * K ** 0.5
+        assert torch.all((got.double() - want).norm(dim=1) <= bound * want.norm(dim=1) + 2e-5 * parts + floor)
+    # beside an infinity and a NaN the other rows keep their values
+    if M > 4:
+        x[1, 5], x[2, 7] = float('inf'), float('nan')
+        again = quantized_matmul(x, qm, transpose_b=True)
+        keep = torch.ones(M, dtype=torch.bool, device='cuda')
+        keep[1] = keep[2] = False
+        assert torch.equal(again[keep], got[keep]) and not torch.isfinite(again[1]).any() and torch.isnan(again[2]).all()
+
+
+@pytest.mark.parametrize('M', [1, 64, 128, 200])
+def test_transposed_matmul_in_the_least_workspace(gg, M):
+    """The least a call is accepted with: whole tiles of 64 rows and four bytes a row, too little for all rows in one
+    pass where M is a multiple of the tile."""
+    from jax_gptq_b200 import _lib
+    lib = _lib.lib
+    K, N = 128, 200
+    g = torch.Generator(device='cuda').manual_seed(M)
+    packed = torch.randint(0, 256, (K // 2, N), generator=g, device='cuda', dtype=torch.uint8)
+    scale, zero = torch.rand(N, generator=g, device='cuda') * 0.01, torch.full((N,), 8.0, device='cuda')
+    x = torch.randn((M, N), generator=g, device='cuda')
+    up = lambda v: (v + 255) // 256 * 256
+    least = 16384 + 2 * up((M + 63) // 64 * 64 * 256 * 2) + up(4 * M)
+    ws = torch.zeros(lib.jgq_w4_matmul_workspace_bytes(M, N, K, 1), dtype=torch.uint8, device='cuda')
+    want = x.double() @ ((torch.stack([packed & 15, packed >> 4], 1).reshape(K, N).double() - 8) * scale.double()).T
+    for nbytes, rc in ((least - 1, -3), (least, 0), (ws.numel(), 0)):
+        out = torch.full((M, K), float('nan'), device='cuda')
+        assert lib.jgq_w4_matmul(x.data_ptr(), _lib.F32, packed.data_ptr(), zero.data_ptr(), scale.data_ptr(), _lib.F32,
+                                 out.data_ptr(), M, N, K, _lib.W4_TRANSPOSE_B, ws.data_ptr(), nbytes, gg._stream()) == rc
+        if rc == 0:
+            assert ((out.double() - want).norm() / want.norm()).item() <= 2e-5
+    assert int(ws[:16384].sum()) == 0
