@@ -197,7 +197,7 @@ __device__ __forceinline__ bool leaf16(const float (*a)[CS], float (*iv)[20], fl
 
 // 64 x 64 tile at (row, col) of a K-stride matrix into registers: thread t holds four consecutive columns
 // 4 (t % 16) of rows t / 16 + 16 q; zeros from row_lim / col_lim on.  `vec`: 16-byte loads are legal.
-__device__ __forceinline__ void tile_fetch(float4 (&v)[4], const float* __restrict__ P, int K, int row, int col,
+__device__ __forceinline__ void tile_fetch(float4 (&v)[4], const float* P, int K, int row, int col,
                                            int row_lim, int col_lim, bool vec) {
   const int t = threadIdx.x, j = col + 4 * (t & 15);
 #pragma unroll
@@ -227,9 +227,10 @@ __device__ __forceinline__ void tile_put(float (*S)[CS], const float4 (&v)[4]) {
 // pivot rows of the inverse X = -iv T, T being the sums P X of the earlier steps; then the rows below take
 // A -= P P^T and T += P X.  R holds the right factors of both updates side by side (P^T, then the pivot rows
 // of X), so that they are one loop.  Warp 0 brings the next pivot block up to date and goes on with it while
-// the other warps finish the update.
+// the other warps finish the update.  (A is not __restrict__: the tile kernel in front may still be writing it when this
+// one starts, which the read-only path that a const __restrict__ pointer allows does not permit.)
 __global__ void __launch_bounds__(256)
-chol_diag_kernel(const float* __restrict__ A, float* __restrict__ X, int K, int kb, int vec,
+chol_diag_kernel(const float* A, float* X, int K, int kb, int vec,
                  int32_t* __restrict__ status) {
   __shared__ __align__(16) float a[CB][CS];
   __shared__ __align__(16) float x[CB][CS];        // T
@@ -387,7 +388,7 @@ __device__ __forceinline__ void tile_mul_nn(float (&acc)[4][4], const float (*U)
 // so that the next diagonal kernel finds a finished block.  With `mirror` the panel tile is also written transposed above
 // the diagonal (A[kb, i], which nothing else uses): the large trailing update reads it there.
 __global__ void __launch_bounds__(256)
-chol_tiles_kernel(float* __restrict__ A, float* __restrict__ X, int K, int kb, int ob, int obe, int tiles_below, int vec, int mirror) {
+chol_tiles_kernel(float* A, float* X, int K, int kb, int ob, int obe, int tiles_below, int vec, int mirror) {
   __shared__ __align__(16) float U[CB][CS];
   __shared__ __align__(16) float V[CB][CS];
   const int r0 = kb * CB;

@@ -252,8 +252,9 @@ w4_gemv_kernel(const __grid_constant__ CUtensorMap wmap, const GemvParams p) {
         for (int h = 0; h < ROWS / 64; ++h) {
           const int k = k0 + 4 * (lane + 32 * h);
           xv[r][h] = XV{};
+          // Not through the read-only path: the previous kernel may write them while this one is already running.
           if (r < p.M && k < p.K)        // K % 8 == 0: the four values are inside the row together
-            xv[r][h] = __ldg(reinterpret_cast<const XV*>((const XT*)p.x + (int64_t)r * p.K + k));
+            xv[r][h] = *reinterpret_cast<const XV*>((const XT*)p.x + (int64_t)r * p.K + k);
         }
     }
     if (alive) alive = __all_sync(0xffffffffu, mbar_wait(&full_bar[slot], (s / GV_NST) & 1, abort_flag));

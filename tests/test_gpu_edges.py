@@ -337,3 +337,28 @@ def test_transposed_matmul_in_the_least_workspace(gg, M):
         if rc == 0:
             assert ((out.double() - want).norm() / want.norm()).item() <= 2e-5
     assert int(ws[:16384].sum()) == 0
+
+
+@pytest.mark.parametrize('dtype', [torch.float16, torch.bfloat16, torch.float32])
+@pytest.mark.parametrize('M', [1, 8, 16])
+def test_matmul_products_that_feed_one_another(gg, M, dtype):
+    """Each product starts while the one that writes its activations is finishing, and the allocator hands the same few
+    buffers around: the bits of the same chain with a synchronisation after every product."""
+    from jax_gptq_b200 import quantized_matmul, QuantizedMatrix
+    K = 1024
+    g = torch.Generator(device='cuda').manual_seed(M)
+    qms = [QuantizedMatrix(torch.randint(0, 256, (K // 2, K), generator=g, device='cuda', dtype=torch.uint8),
+                           torch.full((K,), 7.5, device='cuda'), 0.0065 * (0.9 + 0.2 * torch.rand(K, generator=g, device='cuda'))) for _ in range(4)]
+    x = torch.randn((M, K), generator=g, device='cuda').to(dtype)
+
+    def chain(sync):
+        y = x
+        for i in range(48):
+            y = quantized_matmul(y, qms[i % 4])
+            if sync:
+                torch.cuda.synchronize()
+        return y
+    want = chain(True)
+    assert torch.isfinite(want).all() and want.abs().max() > 0
+    for _ in range(5):
+        assert torch.equal(chain(False), want)
