@@ -284,6 +284,8 @@ def _accumulate_raw(xs, H=None, status=None):
             b = b.contiguous()
         if H is None:
             H = _tmp('H', (K, K), torch.float32, zero=True)
+        elif H.shape[0] != K:
+            raise ValueError(f'a batch of {K} features for a Hessian of {H.shape[0]}')
         n = b.shape[0]
         if not (isinstance(batch, torch.Tensor) and batch.is_cuda and batch.untyped_storage().data_ptr() == b.untyped_storage().data_ptr()):
             size = b.numel() * b.element_size()
@@ -320,6 +322,8 @@ def _accumulate_f64(xs):
             b = b.contiguous()
         if H is None:
             H = torch.zeros((K, K), dtype=torch.float64, device=b.device)
+        elif H.shape[0] != K:
+            raise ValueError(f'a batch of {K} features for a Hessian of {H.shape[0]}')
         check(lib.jgq_hessian_accum_f64(b.data_ptr(), _DT[b.dtype], b.shape[0], K, H.data_ptr(), _stream()))
         n_total += b.shape[0]
     check(lib.jgq_hessian_finalize_f64(H.data_ptr(), H.shape[0], float(n_total), _stream()))

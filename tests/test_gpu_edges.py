@@ -362,3 +362,13 @@ def test_matmul_products_that_feed_one_another(gg, M, dtype):
     assert torch.isfinite(want).all() and want.abs().max() > 0
     for _ in range(5):
         assert torch.equal(chain(False), want)
+
+
+@pytest.mark.parametrize('widths', [(64, 128), (128, 64), (512, 512, 520)])
+@pytest.mark.parametrize('use_fp64', [False, True])
+def test_hessian_refuses_batches_of_another_width(gg, widths, use_fp64):
+    """A wider batch would be added beyond the matrix that the first one was given."""
+    xs = [torch.randn((600, K), device='cuda') for K in widths]
+    with pytest.raises(ValueError, match='features'):
+        gg.accumulate_H(xs, use_fp64=use_fp64)
+    assert torch.isfinite(gg.accumulate_H(xs[:1], use_fp64=use_fp64)).all()
