@@ -31,15 +31,16 @@ def _settled(w):
     return seen == w._version
 
 
-_ws_bytes = {}           # (M, N, K, transpose_b) -> workspace bytes, a function of the sizes alone
+_ws_bytes = {}           # (device, M, N, K, transpose_b) -> workspace bytes: a function of the sizes and the device's SM count
 
 
 def _workspace_bytes(M, N, K, transpose_b):
-    need = _ws_bytes.get((M, N, K, transpose_b))
+    key = (torch.cuda.current_device(), M, N, K, transpose_b)
+    need = _ws_bytes.get(key)
     if need is None:
         if len(_ws_bytes) >= 4096:
             _ws_bytes.clear()
-        need = _ws_bytes[(M, N, K, transpose_b)] = lib.jgq_w4_matmul_workspace_bytes(M, N, K, int(transpose_b))
+        need = _ws_bytes[key] = lib.jgq_w4_matmul_workspace_bytes(M, N, K, int(transpose_b))
     return need
 
 
