@@ -101,7 +101,7 @@ int jgq_col_params(const float* W, int64_t K, int64_t N, int maxq,
  * jgq_hessian_finalize divides by the total sample count and mirrors the
  * lower triangle, giving (1/n) sum x x^T, which accumulate_H returns.
  * dev_status (may be null) receives JGQ_STATUS_LAYOUT if the kernel could not run, JGQ_STATUS_TIMEOUT if a bounded device-side
- * wait of the tensor-core kernel ran out. */
+ * wait of the tensor-core kernel ran out; H is undefined then (start again with a zeroed one). */
 size_t jgq_hessian_workspace_bytes(int64_t n, int64_t K, int x_dtype);
 int jgq_hessian_accum(const void* X, int x_dtype, int64_t n, int64_t K, float* H,
                       void* ws, size_t ws_bytes, int32_t* dev_status, void* stream);

@@ -615,7 +615,8 @@ static void split_planes(const SplitParams& sp, int count, int64_t max_total4, c
 static int launch_pair(HessPairParams& p, int runs, cudaStream_t s) {
   // Test hook for the bounded waits: with JGQ_TEST_WITHHOLD_COMMIT set (read at every launch) the MMA warp keeps its
   // first "chain finished" signal to itself; the waits of every role then run out their budget, the kernel returns
-  // without writing H and reports JGQ_STATUS_TIMEOUT.  Nothing faults and nothing spins without a limit.
+  // and reports JGQ_STATUS_TIMEOUT.  Nothing faults and nothing spins without a limit.  H is undefined after that: tiles and
+  // batches that were complete have been added to it, and slice buffers that were not written are added behind the kernel.
   p.withhold_first_chain = getenv("JGQ_TEST_WITHHOLD_COMMIT") ? 1 : 0;
   struct PairAttrTag {};
   once_per_device<PairAttrTag>([]() {

@@ -372,3 +372,17 @@ def test_hessian_refuses_batches_of_another_width(gg, widths, use_fp64):
     with pytest.raises(ValueError, match='features'):
         gg.accumulate_H(xs, use_fp64=use_fp64)
     assert torch.isfinite(gg.accumulate_H(xs[:1], use_fp64=use_fp64)).all()
+
+
+@pytest.mark.parametrize('K,ns', [(512, (600, 1333, 2048, 777)), (4096, (1024,) * 3)])      # sums by way of buffers, and added to H tile by tile
+def test_hessian_bounded_wait_of_several_batches(gg, K, ns, monkeypatch):
+    """Waits that run out while several batches share a launch: the call raises, H is then undefined, and the next call with
+    a fresh one is correct again."""
+    g = torch.Generator(device='cuda').manual_seed(K)
+    xs = [torch.randn((n, K), generator=g, device='cuda') for n in ns]
+    before = gg.accumulate_H(xs)
+    monkeypatch.setenv('JGQ_TEST_WITHHOLD_COMMIT', '1')
+    with pytest.raises(RuntimeError, match='timed out'):
+        gg.accumulate_H(xs)
+    monkeypatch.delenv('JGQ_TEST_WITHHOLD_COMMIT')
+    assert torch.equal(gg.accumulate_H(xs), before)
