@@ -308,6 +308,31 @@ static size_t w4_forward_need(int64_t M, int64_t N, int64_t K, int x_dtype) {
   return bytes;
 }
 
+// Up to 32 rows: streaming kernel instead of the decode kernel.  A warp of the decode kernel converts a stage's activations
+// for itself, so its time per box grows with rows and planes; a launch of the streaming kernel takes 1 to 5 us more to
+// begin with, more still where many CTAs share a channel group (few channels), and 16 rows at most, but less per box.
+// Measured with weights from HBM, decode / streaming kernel in us:
+//   8192 x 28672   bf16   1 row 44 / 40    8 rows 51 / 46    16 rows 70 / 62    17 rows 135 / 101    32 rows 142 / 122
+//                  f32            51 / 48           82 / 54           143 / 91           191 / 138            286 / 182
+//                  f16            30 / 39           39 / 45            60 / 63           127 /  99            134 / 123
+//   28672 x 8192   bf16           45 / 44           52 / 51            71 / 68           136 / 111            143 / 136
+//   8192 x 14336   bf16           26 / 25           30 / 30            39 / 40            72 /  66             78 /  80
+//                  f32            29 / 29           45 / 34            77 / 53           104 /  82            151 / 104
+//   28672 x 4096   bf16           27 / 30           32 / 37            42 / 50            75 /  86             81 /  96
+//   8192 x 8192    f32            20 / 22           28 / 27            49 / 38            66 /  58             96 /  75
+//                  bf16           18 / 19           21 / 24            27 / 33            46 /  51             52 /  65
+//   4096 x 11008   f32            17 / 19           22 / 22            36 / 31            50 /  49             70 /  61
+//   11008 x 4096   f32            17 / 22           22 / 26            36 / 37            52 /  59             72 /  72
+// Over 493 products on seventeen weight shapes the choice costs 0.2 % over the better kernel.
+static bool w4_streams(int64_t M, int64_t N, int64_t K, int x_dtype) {
+  if ((x_dtype == JGQ_F16 && M <= kStreamRows) || !plan_w4_stream(std::min<int64_t>(M, kStreamRows), N, K).use) return false;
+  const int64_t mi = (N * K) >> 20;
+  if ((N >= 8192 && mi >= 160) || (N >= 12288 && mi >= 96 && M <= 24)) return true;
+  if (x_dtype != JGQ_F32 || M <= 4) return false;
+  if (M <= 8) return (N >= 8192 && mi >= 60) || (N >= 4096 && mi >= 96);
+  return (N >= 8192 && mi >= 40) || mi >= 96;
+}
+
 // Pair kernel or single-CTA kernel, for forward products of more than 32 rows both can run.  Estimates in us, fitted to
 // the GPU time of 9 row counts from 33 to 2048 on seven weight shapes from 768 x 2304 to 8192 x 28672:
 //   single CTA   13 per wave, 0.3 to 0.7 per stage (more with the tile's tokens), 9 per slice of a split contraction and 128
@@ -402,7 +427,7 @@ extern "C" int jgq_w4_matmul(const void* x, int x_dtype, const uint8_t* packed,
   JGQ_REQUIRE(aligned(ws, 256), JGQ_ERR_ALIGN, "w4_matmul: workspace must be 256-byte aligned");
   // Decode sizes: one pass over the weights for all rows, or one per 16 rows (fp32 activations beyond 16; a
   // workspace too small for the slices of 32).  Above 32 rows the tensor-path kernel is the faster one.
-  if (w4_path_override() == 0 && M <= kStreamPassesMaxM && aligned(packed, 16) && aligned(x, 16) && aligned(out, x_dtype == JGQ_F32 ? 16 : 8)) {
+  if (w4_path_override() == 0 && M <= kStreamPassesMaxM && !w4_streams(M, N, K, x_dtype) && aligned(packed, 16) && aligned(x, 16) && aligned(out, x_dtype == JGQ_F32 ? 16 : 8)) {
     const size_t elt = dtype_size(x_dtype);
     for (int64_t step : {M, std::min<int64_t>(M, kStreamRows)}) {
       bool ok = true;
