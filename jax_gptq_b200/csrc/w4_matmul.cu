@@ -333,28 +333,30 @@ static bool w4_streams(int64_t M, int64_t N, int64_t K, int x_dtype) {
   return (N >= 8192 && mi >= 40) || mi >= 96;
 }
 
-// Pair kernel or single-CTA kernel, for forward products of more than 32 rows both can run.  Estimates in us, fitted to
-// the GPU time of 9 row counts from 33 to 2048 on seven weight shapes from 768 x 2304 to 8192 x 28672:
-//   single CTA   13 per wave, 0.3 to 0.7 per stage (more with the tile's tokens), 9 per slice of a split contraction and 128
-//                tokens for the slices' exchange;
+// Pair kernel or single-CTA kernel, for forward products of more than 32 rows both can run: the smaller of two estimates in
+// us, each fitted (least squares of the logarithm, 5 % rms) to that kernel's GPU time at eleven row counts from 33 to 512 on
+// fifteen weight shapes from 256 x 14544 and 768 x 768 to 8192 x 28672, per number of activation planes:
+//   single CTA   per wave of CTAs its stages (more with the tile's tokens) and an epilogue, the exchange of the slices of a split
+//                contraction, the kernel in front;
 //   pair         see plan_w4_pair.
-// The single-CTA kernel keeps few rows on long contractions (64 rows, K = 11008, N = 4096: 76 against 82 us; 128 rows of
-// fp32: 87 against 133); more than 256 rows of 16-bit activations always go to the pairs (2048 rows, 4096 x 11008: 293
-// against 176 us).  The transposed product takes the pairs whenever they can run (33 rows, 4096 x 4096: 108 against
-// 53 us; 2048 rows, 11008 x 4096: 894 against 276).
+// On those 495 products the choice costs 0.1 % over the better kernel, 5 % at worst.  Examples, single CTA / pair:
+// 64 rows of f16, 4096 x 4096: 35 / 38 us; 96 rows: 45 / 39; 192 rows, 11008 x 4096: 92 / 99; 64 rows of fp32, 8192 x 8192: 97 / 78.
+// More than 512 rows of 16-bit activations always go to the pairs (2048 rows, 4096 x 11008: 293 / 176).
+// The transposed product takes the pairs whenever they can run.  mma.sync kernel / pairs: 33 rows, 4096 x 4096: 106 / 36 us; few
+// outputs and a long contraction, K x N = 64 x 32000: 1 row 639 / 226, 2048 rows 1135 / 476; 11008 x 256: 23 / 16 and 85 / 46.
 static PairPlan w4_pair_choice(int64_t M, int64_t N, int64_t K, int x_dtype, int transpose_b) {
   const int ov = w4_path_override();
   PairPlan pp = plan_w4_pair(M, N, K, x_dtype, transpose_b);
   if (!pp.use || ov != 0 || transpose_b) { pp.use = pp.use && ov == 0; return pp; }
   if (M <= kStreamPassesMaxM) { pp.use = 0; return pp; }
-  if (pp.planes == 1 && M > 256) return pp;
+  if (pp.planes == 1 && M > 512) return pp;
   const UmmaPlan up = plan_w4_umma(M, N, K, x_dtype);
   if (!up.use) return pp;
-  const int sms = sm_count();
-  const double stage = up.planes == 2 ? 0.35 + 0.0022 * up.NT : 0.3 + 0.0016 * up.NT;
-  const double single = (double)cdiv((int64_t)up.ncg * up.mtiles * up.ksplit, sms) * (stage * up.stages_per_split + 13.0) +
-                        (up.ksplit > 1 ? 9.0 / 128.0 * up.NT * up.ksplit : 0.0);
-  pp.use = pp.us < 0.93 * (single + 10.0);
+  const double waves = (double)cdiv((int64_t)up.ncg * up.mtiles * up.ksplit, sm_count());
+  const double exchange = up.ksplit > 1 ? (double)up.NT * up.ksplit : 0.0, rows = (double)M / 256;
+  const double single = up.planes == 2 ? 6.0 + waves * ((0.461 + 0.00056 * up.NT) * up.stages_per_split + 1.4 + 0.061 * up.NT) + 0.062 * exchange + 2.0 * rows
+                                       : 1.6 + waves * ((0.378 + 0.0009 * up.NT) * up.stages_per_split + 4.3 + 0.047 * up.NT) + 0.056 * exchange + 7.3 * rows;
+  pp.use = pp.us < single;
   return pp;
 }
 

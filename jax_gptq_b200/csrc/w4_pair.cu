@@ -437,10 +437,12 @@ PairPlan plan_w4_pair(int64_t M, int64_t N, int64_t K, int x_dtype, int transpos
   pl.cols = (int)(pl.planes == 2 ? 0 : cols / 2 * 2);
   pl.items = (int)(pl.twos + pl.halves + odd);
   pl.G = std::min(pairs, pl.items);
-  // a stage takes 0.43 us with one block of tokens, 0.68 with two
-  const double nst = (double)cdiv(pl.depth, P_STAGE_K), one = (pl.planes == 2 ? 0.70 : 0.43) * nst + 2.0, two = 0.68 * nst + 4.0;
+  // Estimate of the forward product (see w4_pair_choice): per round the stages and the outputs of a tile, more with its
+  // tokens; 0.68 us a stage for two tiles at once.
+  const double nst = (double)cdiv(pl.depth, P_STAGE_K), nt = pl.nt, two = 0.68 * nst + 4.0;
+  const double one = pl.planes == 2 ? (0.50 + 0.00069 * nt) * nst + 0.0168 * nt : (0.475 + 0.00028 * nt) * nst + 0.0121 * nt;
   const int64_t rounds = cdiv(pl.twos, pairs), room = rounds * pairs - pl.twos;
-  pl.us = (double)rounds * two + (double)cdiv(std::max<int64_t>(0, pl.halves + odd - room), pairs) * one + 12.0;
+  pl.us = (double)rounds * two + (double)cdiv(std::max<int64_t>(0, pl.halves + odd - room), pairs) * one + (pl.planes == 2 ? 7.2 : 5.9);
   pl.Np = cdiv(N, P_STAGE_K) * P_STAGE_K;
   pl.plane_bytes = pl.planes == 1 ? 0 : align_up((size_t)M * (transpose_b ? pl.Np : K) * 2, 256);
   pl.tok_bytes = align_up((size_t)M * (transpose_b ? sizeof(float2) : sizeof(float)), 256);
