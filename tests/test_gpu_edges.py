@@ -148,9 +148,10 @@ def test_matmul_decode_rows_types_and_ragged_edges(gg, M, dtype, K, N):
         first = got
 
 
-@pytest.mark.parametrize('M,dtype', [(24, torch.float16), (32, torch.bfloat16), (12, torch.float32), (20, torch.float32)])
-def test_matmul_with_the_smallest_workspace_it_accepts(gg, M, dtype):
-    """The slices of 32 rows are larger than what a call is refused without; with a smaller workspace it takes two passes."""
+@pytest.mark.parametrize('M,dtype,passes', [(24, torch.float16, 2), (32, torch.bfloat16, 2), (12, torch.float32, 1), (20, torch.float32, 2)])
+def test_matmul_with_the_smallest_workspace_it_accepts(gg, M, dtype, passes):
+    """The slices of 32 rows are larger than what a call is refused without; with the least workspace 16-bit activations
+    take the decode kernel in passes of 16 rows: the bits of separate calls for those rows."""
     from jax_gptq_b200 import _lib
     lib = _lib.lib
     N, K = 2048, 8192
@@ -159,19 +160,35 @@ def test_matmul_with_the_smallest_workspace_it_accepts(gg, M, dtype):
     scale, zero = torch.rand(N, generator=g, device='cuda') * 0.01, torch.full((N,), 8.0, device='cuda')
     x = torch.randn((M, K), generator=g, device='cuda').to(dtype)
     full = lib.jgq_w4_matmul_workspace_bytes(M, N, K, 0)
-    outs = []
     ws = torch.zeros(full, dtype=torch.uint8, device='cuda')
-    for nbytes in (full, full // 2, full // 4, full // 8):
-        out = torch.full((M, N), float('nan'), dtype=dtype, device='cuda')
-        rc = lib.jgq_w4_matmul(x.data_ptr(), gg._DT[dtype], packed.data_ptr(), zero.data_ptr(), scale.data_ptr(), _lib.F32,
-                               out.data_ptr(), M, N, K, 0, ws.data_ptr(), nbytes, gg._stream())
-        if rc == -3:
-            continue
-        assert rc == 0
-        outs.append(out)
+
+    def call(rows, nbytes):
+        out = torch.full((rows.shape[0], N), float('nan'), dtype=dtype, device='cuda')
+        before = lib.jgq_launch_count()
+        rc = lib.jgq_w4_matmul(rows.data_ptr(), gg._DT[dtype], packed.data_ptr(), zero.data_ptr(), scale.data_ptr(), _lib.F32,
+                               out.data_ptr(), rows.shape[0], N, K, 0, ws.data_ptr(), nbytes, gg._stream())
+        assert rc in (0, -3)
+        return (out, lib.jgq_launch_count() - before) if rc == 0 else None
+    refused, least = 0, full
+    while least - refused > 1:
+        mid = (least + refused) // 2
+        if call(x, mid) is None:
+            refused = mid
+        else:
+            least = mid
     want = x.double() @ ((torch.stack([packed & 15, packed >> 4], 1).reshape(K, N).double() - 8) * scale.double())
-    for out in outs:
-        assert ((out.double() - want).norm() / want.norm()).item() <= {torch.float16: 2.0 ** -11, torch.bfloat16: 2.0 ** -8, torch.float32: 2e-5}[dtype]
+    bound = {torch.float16: 2.0 ** -11, torch.bfloat16: 2.0 ** -8, torch.float32: 2e-5}[dtype]
+    for nbytes in (least, least + 256, full):
+        out, launches = call(x, nbytes)
+        assert ((out.double() - want).norm() / want.norm()).item() <= bound
+        if nbytes <= least + 256:
+            assert launches == passes
+            if dtype != torch.float32:
+                assert least < full
+                assert torch.equal(out, torch.cat([call(x[:16], full)[0], call(x[16:], full)[0]]))
+        elif dtype != torch.float32:
+            assert launches == 1
+    assert call(x, least - 1) is None
     assert int(ws[:16384].sum()) == 0                    # the tickets are back at zero
 
 
@@ -386,3 +403,60 @@ def test_hessian_bounded_wait_of_several_batches(gg, K, ns, monkeypatch):
         gg.accumulate_H(xs)
     monkeypatch.delenv('JGQ_TEST_WITHHOLD_COMMIT')
     assert torch.equal(gg.accumulate_H(xs), before)
+
+
+@pytest.mark.parametrize('parity', [0, 1])
+def test_damp_invert_roots_and_reciprocals_of_many_mantissas(gg, parity):
+    """A diagonal matrix is factored pivot by pivot: the factor of its inverse is 1 / sqrt, both operations IEEE's, bit for
+    bit; every 32nd mantissa, the neighbours of the powers of two, and pivots whose root has the largest mantissa, in both
+    exponent parities, and the values at which the fast form hands over to the plain one."""
+    K = 4096
+    m = np.concatenate([np.arange(parity, 1 << 23, 32), np.arange(64), (1 << 23) - 1 - np.arange(64)]).astype(np.uint32)
+    a = (m | np.uint32((127 + parity) << 23)).view(np.float32)
+    edge = np.float32([2.0 ** -96, 2.0 ** 96, np.nextafter(np.float32(2.0 ** -96), np.float32(0)), np.nextafter(np.float32(2.0 ** 96), np.float32(np.inf)), 1e-37, 1e37])
+    a = np.concatenate([a, edge, np.ones(-(len(a) + len(edge)) % K, np.float32)])
+    want = np.float32(1) / np.sqrt(a)
+    W = torch.zeros((K, 1), device='cuda')
+    for s in range(0, len(a), K):
+        L, status = gg._damp_and_invert(W, torch.diag(dev(a[s:s + K])), 0.0)
+        assert int(status.item()) == 0
+        assert np.array_equal(torch.diagonal(L).cpu().numpy(), want[s:s + K])
+    assert torch.count_nonzero(L) == K
+
+
+def test_matmul_tensor_path_on_the_single_cta_kernel():
+    """Which tensor-core kernel a product takes depends on its sizes.  With JGQ_W4_PATH=stream, read once per process, more
+    than 32 rows all take the single-CTA kernel: the ring depths, split contractions, two planes and launches of hundreds of
+    CTAs that `test_matmul_tensor_path_every_channel_group` and `test_matmul_many_ctas_repeatable` list, in a process of its own."""
+    import os
+    import subprocess
+    import sys
+    here = os.path.dirname(os.path.abspath(__file__))
+    r = subprocess.run([sys.executable, '-m', 'pytest', '-q', '-x', '-p', 'no:cacheprovider', os.path.join(here, 'test_gpu_parity.py'),
+                        '-k', 'every_channel_group or many_ctas_repeatable'], env=dict(os.environ, JGQ_W4_PATH='stream'),
+                       capture_output=True, text=True, timeout=900)
+    assert r.returncode == 0, r.stdout[-3000:]
+    assert '11 passed' in r.stdout
+
+
+@pytest.mark.parametrize('M,K,N,dtype', [(9, 5120, 8192, torch.float32), (9, 5112, 8192, torch.float32), (16, 5128, 8208, torch.float32),
+                                         (5, 7680, 8192, torch.float32), (4, 7680, 8192, torch.float32), (32, 24576, 4096, torch.float32),
+                                         (8, 24584, 4096, torch.float32), (17, 8192, 12288, torch.float16), (16, 8192, 12288, torch.float16),
+                                         (24, 8200, 12304, torch.bfloat16), (25, 8192, 12288, torch.bfloat16), (1, 8192, 20480, torch.bfloat16),
+                                         (32, 20488, 8192, torch.float16)])
+def test_matmul_decode_rows_of_large_weights(gg, M, K, N, dtype):
+    """Both sides of the lines between the decode kernel and the streaming kernel, against the dequantized product in fp64:
+    the output's rounding, or the planes' 2^-17 and fp32 sums.  f16 activations of 1e-4 among them."""
+    from jax_gptq_b200 import quantized_matmul, QuantizedMatrix
+    g = torch.Generator(device='cuda').manual_seed(M + K + N)
+    packed = torch.randint(0, 256, (K // 2, N), generator=g, device='cuda', dtype=torch.uint8)
+    scale = 0.001 + 0.019 * torch.rand(N, generator=g, device='cuda')
+    zero = torch.randint(0, 16, (N,), generator=g, device='cuda').float()
+    x = (torch.randn((M, K), generator=g, device='cuda') * torch.tensor([1.0, 1e-4], device='cuda')[torch.arange(M, device='cuda') % 2][:, None]).to(dtype)
+    got = quantized_matmul(x, QuantizedMatrix(packed, zero, scale))
+    assert torch.equal(got, quantized_matmul(x, QuantizedMatrix(packed, zero, scale)))
+    bound = {torch.float16: 2.0 ** -11, torch.bfloat16: 2.0 ** -8, torch.float32: 2e-5}[dtype]
+    for c in range(0, N, 2048):
+        w = packed[:, c:c + 2048]
+        want = x.double() @ ((torch.stack([w & 15, w >> 4], 1).reshape(K, -1).double() - zero[c:c + 2048].double()) * scale[c:c + 2048].double())
+        assert torch.all((got[:, c:c + 2048].double() - want).norm(dim=1) <= bound * want.norm(dim=1))

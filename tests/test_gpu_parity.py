@@ -594,7 +594,7 @@ def test_matmul_many_ctas_repeatable(G, M, x_dtype):
 
 @pytest.mark.parametrize('M,N,K,x_dtype,rings', [
     (64, 32000, 5120, 'float16', None),          # 80 stages per CTA, eight expansion warps
-    (600, 8192, 5120, 'float16', None),          # 512-token tiles: both accumulators, four expansion slots
+    (600, 8192, 5120, 'float16', None),          # 256-token tiles: four expansion slots
     (100, 4096, 5120, 'float32', None),          # two activation planes
     (48, 1024, 8192, 'bfloat16', None),          # few channel groups: split-K with tickets
     (64, 16384, 5120, 'float16', '8,4,2'),       # two warps per stage, a two-deep activation ring
@@ -602,10 +602,11 @@ def test_matmul_many_ctas_repeatable(G, M, x_dtype):
     (128, 16384, 2560, 'float16', '8,8,3'),      # a raw ring no deeper than the expansion warps
 ])
 def test_matmul_tensor_path_every_channel_group(G, M, N, K, x_dtype, rings, monkeypatch):
-    """The tensor-core kernel against an independent product (fp32 matmul of the unpacked weights), judged
+    """The tensor-core kernels against an independent product (fp32 matmul of the unpacked weights), judged
     per 128-channel group - one CTA's work - so that a single CTA with a few per cent of wrong sums cannot
-    hide in the norm of the whole output; ring depths, warps per stage, split-K, two planes and the
-    two-accumulator tile are all visited.  Five launches must agree bit for bit."""
+    hide in the norm of the whole output.  Five launches must agree bit for bit.  The cases name what they are to the
+    single-CTA kernel (ring depths, warps per stage, split-K, two planes), which takes them all with JGQ_W4_PATH=stream, as
+    `test_matmul_tensor_path_on_the_single_cta_kernel` runs them; without it most go to the CTA-pair kernel."""
     if rings:
         monkeypatch.setenv('JGQ_UMMA_RINGS', rings)
     torch.manual_seed(7)
