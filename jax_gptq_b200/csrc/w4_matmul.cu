@@ -353,9 +353,10 @@ static PairPlan w4_pair_choice(int64_t M, int64_t N, int64_t K, int x_dtype, int
   const UmmaPlan up = plan_w4_umma(M, N, K, x_dtype);
   if (!up.use) return pp;
   const double waves = (double)cdiv((int64_t)up.ncg * up.mtiles * up.ksplit, sm_count());
-  const double exchange = up.ksplit > 1 ? (double)up.NT * up.ksplit : 0.0, rows = (double)M / 256;
-  const double single = up.planes == 2 ? 6.0 + waves * ((0.461 + 0.00056 * up.NT) * up.stages_per_split + 1.4 + 0.061 * up.NT) + 0.062 * exchange + 2.0 * rows
-                                       : 1.6 + waves * ((0.378 + 0.0009 * up.NT) * up.stages_per_split + 4.3 + 0.047 * up.NT) + 0.056 * exchange + 7.3 * rows;
+  const double exchange = up.ksplit > 1 ? up.ksplit : 0.0, rows = (double)M / 256;      // per slice: its tile's tokens
+  const double single = up.planes == 2 ? 6.0 + waves * ((0.461 + 0.00056 * up.NT) * up.stages_per_split + 1.4 + 0.061 * up.NT) + 0.062 * exchange * up.NT + 2.0 * rows
+                                       : 3.1 + waves * ((0.3943 + 0.0007 * up.NT) * up.stages_per_split + 3.26 + 0.0544 * up.NT) +
+                                             0.0598 * exchange * (double)(up.mtiles == 1 ? M : up.NT) + 3.9 * rows;
   pp.use = pp.us < single;
   return pp;
 }
