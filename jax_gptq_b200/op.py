@@ -14,10 +14,11 @@ from torch.autograd import forward_ad
 
 from . import _lib
 from ._lib import lib, check
-from .gptq import _to_dev, _out, _is_np, _stream, _workspace, _DT
+from .gptq import _to_dev, _out, _is_np, _workspace, _DT
 
 _functorch_active = torch._C._functorch.peek_interpreter_stack
 _tracing = torch._C._get_tracing_state
+_current_device, _raw_stream = torch._C._cuda_getDevice, torch._C._cuda_getCurrentRawStream     # the context exists by then
 _ZS = {torch.float32: _lib.F32, torch.float16: _lib.F16}
 
 
@@ -34,8 +35,9 @@ def _settled(w):
 _ws_bytes = {}           # (device, M, N, K, transpose_b) -> workspace bytes: a function of the sizes and the device's SM count
 
 
-def _workspace_bytes(M, N, K, transpose_b):
-    key = (torch.cuda.current_device(), M, N, K, transpose_b)
+def _workspace_bytes(dev, M, N, K, transpose_b):
+    """For the current device, whose index is `dev`."""
+    key = (dev, M, N, K, transpose_b)
     need = _ws_bytes.get(key)
     if need is None:
         if len(_ws_bytes) >= 4096:
@@ -56,11 +58,12 @@ def _launch(x, w, zero, scale, transpose_b):
     K2, out_n = (Nw, Kw) if transpose_b else (Kw, Nw)    # op.py:30-40
     assert K == K2, f'Inner dim mismatch: {K} != {K2}'   # op.py:41
     out = x.new_empty((M, out_n))
-    need = _workspace_bytes(M, Nw, Kw, transpose_b)
+    dev = _current_device()
+    need = _workspace_bytes(dev, M, Nw, Kw, transpose_b)
     ws = _workspace(need, zeroed=True, tag='w4').data_ptr() if need else 0
     flags = (_lib.W4_TRANSPOSE_B if transpose_b else 0) | (_lib.W4_WEIGHTS_SETTLED if _settled(w) else 0)
     rc = lib.jgq_w4_matmul(x.data_ptr(), _DT[x.dtype], w.data_ptr(), zero.data_ptr(), scale.data_ptr(),
-                           _ZS[zero.dtype], out.data_ptr(), M, Nw, Kw, flags, ws, need, _stream())
+                           _ZS[zero.dtype], out.data_ptr(), M, Nw, Kw, flags, ws, need, _raw_stream(dev))
     if rc:
         check(rc)
     return out if len(shape) == 2 else out.reshape(shape[:-1] + (out_n,))

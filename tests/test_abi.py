@@ -65,15 +65,13 @@ def test_validation_errors_without_gpu(jlib):
 def test_matmul_workspace_size_is_kept_per_device(jlib, monkeypatch):
     """The plans behind the size count the SMs of the current device: one looked up on one device is not another's."""
     import types
-    import torch
     from jax_gptq_b200 import op
     device = 0
-    monkeypatch.setattr(torch.cuda, 'current_device', lambda: device)
     monkeypatch.setattr(op, 'lib', types.SimpleNamespace(jgq_w4_matmul_workspace_bytes=lambda M, N, K, t: 1000 * (device + 1) + t))
     monkeypatch.setattr(op, '_ws_bytes', {})
-    assert op._workspace_bytes(8, 64, 64, False) == 1000
+    assert op._workspace_bytes(0, 8, 64, 64, False) == 1000
     device = 1
-    assert op._workspace_bytes(8, 64, 64, False) == 2000
-    assert op._workspace_bytes(8, 64, 64, True) == 2001
+    assert op._workspace_bytes(1, 8, 64, 64, False) == 2000
+    assert op._workspace_bytes(1, 8, 64, 64, True) == 2001
     device = 0
-    assert op._workspace_bytes(8, 64, 64, False) == 1000
+    assert op._workspace_bytes(0, 8, 64, 64, False) == 1000
