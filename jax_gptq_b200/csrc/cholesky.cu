@@ -15,7 +15,7 @@
 //
 // (4) and (5) run once per outer block of four panels, with depth 256; inside an outer block
 // (2) and (3) apply the block's earlier panels to their tiles themselves.  S lives in the
-// not-yet-final part of X.  Everything is fp32 with IEEE division and square root.
+// not-yet-final part of X.  Everything is fp32; roots and quotients are rounded as IEEE's are.
 #include "common.cuh"
 #include <algorithm>
 #include <cstdlib>
@@ -88,8 +88,9 @@ __global__ void zero_dead_rows_kernel(float* __restrict__ W, int K, int64_t N,
 constexpr int CS = CB + 4;      // row stride of the shared 64 x 64 tiles: 16-byte rows, eight rows on 32 banks
 
 // d = sqrt(a) and y = 1 / d, both rounded to nearest, for a in [2^-96, 2^96]: Goldschmidt iterations on the
-// hardware's reciprocal root with the residual corrections of Markstein (IBM J. R&D 34, 1990).  Checked
-// against the IEEE operations over every mantissa and both exponent parities: d always, y but for d's largest mantissa.  About 70 cycles for the
+// hardware's reciprocal root with the residual corrections of Markstein (IBM J. R&D 34, 1990).  Equal to the IEEE
+// operations for every mantissa and both exponent parities, d always, y but for d's largest mantissa, which leaf16 gives to
+// the plain operations (compared through the factorization of diagonal matrices; the tests repeat every 32nd mantissa).  About 70 cycles for the
 // pair; an IEEE root takes 55, and each division by it 50 more where divide_by takes 20.
 __device__ __forceinline__ void root_and_reciprocal(float a, float& d, float& y) {
   float h, g, e;

@@ -261,7 +261,10 @@ static int launch_fwd(const void* x, const uint8_t* packed, const void* zero, co
 }
 
 constexpr int64_t kStreamRows = 16;          // token rows of one pass of the streaming kernel
-constexpr int64_t kStreamPassesMaxM = 32;    // two passes (120 us at 8192 x 28672) still beat the tensor-path kernel (128 us at M = 64)
+// Rows up to which the decode or the streaming kernel takes a product, against the tensor-path kernels (32 rows against
+// 33): f16 768 x 2304 12.3 / 12.0 us, 11008 x 4096 39 / 53, 8192 x 8192 50 / 69, 8192 x 28672 123 / 119; fp32 11008 x 4096 72 / 60,
+// 8192 x 28672 182 / 133 (with fp32 activations, two planes in passes of 16 rows, the line would be better below 32).
+constexpr int64_t kStreamPassesMaxM = 32;
 
 static int w4_path_override() {        // JGQ_W4_PATH=direct: direct-load decode kernel; =mma: no tcgen05 either; =stream: no decode kernel
   static const int v = []() {

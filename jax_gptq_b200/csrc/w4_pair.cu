@@ -36,9 +36,10 @@
 // (bytes of both CTAs' loads) and acc_empty (arrivals of both CTAs' epilogue warps) live in the even CTA; a_empty, x_empty
 // and acc_full exist in both and are signalled by two commits each.  No load uses multicast.  Waits are bounded: a timed-out product writes NaN.
 //
-// Measured (call to call): forward, 2048 x 4096 x 11008, bf16: 291 us on the single-CTA kernel, 177 with a tile per pair and
-// launch, 156 now, 1.19 PFLOP/s (of 1.67 measured with cuBLAS in a burst); transposed, 2048 rows on 11008 x 4096: 894 with
-// mma.sync, 275, 241, 1.53 PFLOP/s executed for two planes; 512 rows, 11008 x 4096: 137 -> 98.  Up to 256 rows of 16-bit
+// Measured (replayed over rotating weights): forward, 2048 x 4096 x 11008, bf16: 291 us on the single-CTA kernel, 177 with a
+// tile per pair and launch, 152 now, 1.22 PFLOP/s (of 1.67 measured with cuBLAS in a burst; 175 us in a loop of calls that
+// changes its inputs); transposed, 2048 rows on 11008 x 4096: 894 with mma.sync, 275, 244, 1.52 PFLOP/s executed for two
+// planes; 512 rows, 11008 x 4096: 137 -> 98.  Up to 256 rows of 16-bit
 // activations, where a pair has one or two items, it is even or up to 7 % slower than a tile per launch (256 rows, 11008 x 4096:
 // 88 -> 95 us).
 // Without the MMAs a stage takes 0.38 us, with them 0.68: the tensor pipe and the
