@@ -460,3 +460,32 @@ def test_matmul_decode_rows_of_large_weights(gg, M, K, N, dtype):
         w = packed[:, c:c + 2048]
         want = x.double() @ ((torch.stack([w & 15, w >> 4], 1).reshape(K, -1).double() - zero[c:c + 2048].double()) * scale[c:c + 2048].double())
         assert torch.all((got[:, c:c + 2048].double() - want).norm(dim=1) <= bound * want.norm(dim=1))
+
+
+@pytest.mark.parametrize('M,N', [(150, 1024), (150, 1040), (300, 2048), (300, 2064), (149, 4096), (148, 4096), (149, 4112), (2, 8192), (3, 8208), (150, 16400), (150, 1025)])
+@pytest.mark.parametrize('dtype,zs', [(torch.bfloat16, torch.float32), (torch.float32, torch.float16)])
+@pytest.mark.parametrize('shift', [0, 1])
+def test_transposed_matmul_rows_of_any_length_and_alignment(gg, M, N, dtype, zs, shift):
+    """Row lengths and counts at which the kernel in front changes its block, rows that it keeps in registers and longer ones;
+    activations, scales and zero points that do not start on 16 bytes (or on 8)."""
+    from jax_gptq_b200 import quantized_matmul, QuantizedMatrix
+    K = 64
+    g = torch.Generator(device='cuda').manual_seed(M + N)
+
+    def moved(t):
+        flat = torch.zeros(t.numel() + 16, dtype=t.dtype, device='cuda')
+        flat[shift:shift + t.numel()] = t.reshape(-1)
+        return flat[shift:shift + t.numel()].view(t.shape)
+    packed = torch.randint(0, 256, (K // 2, N), generator=g, device='cuda', dtype=torch.uint8)
+    scale = moved((0.001 + 0.019 * torch.rand(N, generator=g, device='cuda')).to(zs))
+    zero = moved(torch.randint(0, 16, (N,), generator=g, device='cuda').to(zs))
+    x = moved((torch.randn((M, N), generator=g, device='cuda') * 1e-5).to(dtype))
+    codes = torch.stack([packed & 15, packed >> 4], 1).reshape(K, N).double()
+    want = x.double() @ ((codes - zero.double()) * scale.double()).T
+    parts = x.double() @ (codes * scale.double()).T                        # sums of the codes and of the zero points, apart
+    got = quantized_matmul(x, QuantizedMatrix(packed, zero, scale), transpose_b=True).double()
+    # fp32 sums in one chain over N: a tensor core drops what lies below the accumulator's last bit at each of N / 16 steps
+    # (two planes: N / 8), at most 2^-23 of it, half of that on average; the accumulator grows with the steps: N / 8 x 2^-25 of its end
+    bound = {torch.bfloat16: 2.0 ** -8, torch.float32: 0.0}[dtype]
+    sums = max(2e-5, N / 8 * 2.0 ** -25)
+    assert torch.all((got - want).norm(dim=1) <= bound * want.norm(dim=1) + sums * (parts.norm(dim=1) + (parts - want).norm(dim=1)))
