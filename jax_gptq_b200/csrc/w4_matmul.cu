@@ -263,7 +263,7 @@ static int launch_fwd(const void* x, const uint8_t* packed, const void* zero, co
 constexpr int64_t kStreamRows = 16;          // token rows of one pass of the streaming kernel
 // Rows up to which the decode or the streaming kernel takes a product, against the tensor-path kernels (32 rows against
 // 33): f16 768 x 2304 12.3 / 12.0 us, 11008 x 4096 39 / 53, 8192 x 8192 50 / 69, 8192 x 28672 123 / 119; fp32 11008 x 4096 72 / 60,
-// 8192 x 28672 182 / 133 (with fp32 activations, two planes in passes of 16 rows, the line would be better below 32).
+// 8192 x 28672 187 / 133 (with fp32 activations, two planes in passes of 16 rows, the line would be better below 32).
 constexpr int64_t kStreamPassesMaxM = 32;
 
 static int w4_path_override() {        // JGQ_W4_PATH=direct: direct-load decode kernel; =mma: no tcgen05 either; =stream: no decode kernel
@@ -316,22 +316,24 @@ static size_t w4_forward_need(int64_t M, int64_t N, int64_t K, int x_dtype) {
 // begin with, more still where many CTAs share a channel group (few channels), and 16 rows at most, but less per box.
 // Measured with weights from HBM, decode / streaming kernel in us:
 //   8192 x 28672   bf16   1 row 44 / 40    8 rows 51 / 46    16 rows 70 / 62    17 rows 135 / 101    32 rows 142 / 122
-//                  f32            51 / 48           82 / 54           143 / 91           191 / 138            286 / 182
+//                  f32            51 / 50           81 / 57           143 / 92           192 / 142            285 / 187
 //                  f16            30 / 39           39 / 45            60 / 63           127 /  99            134 / 123
 //   28672 x 8192   bf16           45 / 44           52 / 51            71 / 68           136 / 111            143 / 136
+//                  f32            52 / 54           83 / 66           145 / 98           194 / 153            290 / 203
 //   8192 x 14336   bf16           26 / 25           30 / 30            39 / 40            72 /  66             78 /  80
-//                  f32            29 / 29           45 / 34            77 / 53           104 /  82            151 / 104
+//                  f32            29 / 30           45 / 36            77 / 55           104 /  84            152 / 106
 //   28672 x 4096   bf16           27 / 30           32 / 37            42 / 50            75 /  86             81 /  96
-//   8192 x 8192    f32            20 / 22           28 / 27            49 / 38            66 /  58             96 /  75
+//   8192 x 8192    f32            20 / 22           28 / 27            49 / 39            66 /  60             96 /  76
 //                  bf16           18 / 19           21 / 24            27 / 33            46 /  51             52 /  65
-//   4096 x 11008   f32            17 / 19           22 / 22            36 / 31            50 /  49             70 /  61
+//   4096 x 11008   f32            17 / 19           22 / 22            36 / 32            50 /  50             70 /  62
 //   11008 x 4096   f32            17 / 22           22 / 26            36 / 37            52 /  59             72 /  72
 // Over 493 products on seventeen weight shapes the choice costs 0.2 % over the better kernel.
 static bool w4_streams(int64_t M, int64_t N, int64_t K, int x_dtype) {
   if ((x_dtype == JGQ_F16 && M <= kStreamRows) || !plan_w4_stream(std::min<int64_t>(M, kStreamRows), N, K).use) return false;
   const int64_t mi = (N * K) >> 20;
-  if ((N >= 8192 && mi >= 160) || (N >= 12288 && mi >= 96 && M <= 24)) return true;
-  if (x_dtype != JGQ_F32 || M <= 4) return false;
+  const bool f32 = x_dtype == JGQ_F32;
+  if ((N >= (f32 && M <= 4 ? 12288 : 8192) && mi >= 160) || (N >= 12288 && mi >= 96 && M <= 24)) return true;
+  if (!f32 || M <= 4) return false;
   if (M <= 8) return (N >= 8192 && mi >= 60) || (N >= 4096 && mi >= 96);
   return (N >= 8192 && mi >= 40) || mi >= 96;
 }
@@ -342,8 +344,8 @@ static bool w4_streams(int64_t M, int64_t N, int64_t K, int x_dtype) {
 //   single CTA   per wave of CTAs its stages (more with the tile's tokens) and an epilogue, the exchange of the slices of a split
 //                contraction, the kernel in front;
 //   pair         see plan_w4_pair.
-// On those 495 products the choice costs 0.1 % over the better kernel, 5 % at worst.  Examples, single CTA / pair:
-// 64 rows of f16, 4096 x 4096: 35 / 38 us; 96 rows: 45 / 39; 192 rows, 11008 x 4096: 92 / 99; 64 rows of fp32, 8192 x 8192: 97 / 78.
+// On those 495 products the estimates choose within 0.1 % of the better kernel, 5 % at worst.  Examples, single CTA / pair:
+// 64 rows of f16, 4096 x 4096: 35 / 38 us; 96 rows: 45 / 39; 192 rows, 11008 x 4096: 92 / 99; 160 rows of fp32, 4096 x 11008: 85 / 51.
 // More than 512 rows of 16-bit activations always go to the pairs (2048 rows, 4096 x 11008: 293 / 176).
 // The transposed product takes the pairs whenever they can run.  mma.sync kernel / pairs: 33 rows, 4096 x 4096: 106 / 36 us; few
 // outputs and a long contraction, K x N = 64 x 32000: 1 row 639 / 226, 2048 rows 1135 / 476; 11008 x 256: 23 / 16 and 85 / 46.

@@ -13,7 +13,8 @@
 // and the high nibble of one byte into the two halves, and one logic operation (and-mask,
 // or-exponent, both constants held as kernel parameters).  The operand then reads
 // OFFSET + code (64 for f16, 128 for bf16); the offset is folded into the zero point,
-// out = scale * (acc - (zero + OFFSET) * sum_k x), with sum_k x from an MMA against ones.
+// out = scale * (acc - (zero + OFFSET) * sum_k x), with sum_k x from an MMA against ones (fp32
+// activations: taken off the operand again, see unbiased; 4 % of the time).
 //
 // The grid is one resident wave.  Work is the list of all stages, ordered by (channel group,
 // contraction position); CTA c owns the contiguous range [c*S/G, (c+1)*S/G) of it, so every
@@ -91,6 +92,16 @@ template <> struct Biased<__nv_bfloat16> {
     return (__byte_perm(w, o, sel) & mask) | magic;
   }
 };
+// fp32 activations (two planes): the offset is taken off again on the FMA pipe.  Folded into the zero point, sums of 128 + code lose
+// bits that an fp32 result keeps (relative error 4e-6 to 5e-6; without the offset 2.4e-6, most of it the planes').
+template <typename CT, bool kSplitX>
+__device__ __forceinline__ uint32_t unbiased(uint32_t a) {
+  if constexpr (kSplitX) {
+    const __nv_bfloat162 h = __hsub2(*reinterpret_cast<const __nv_bfloat162*>(&a), __float2bfloat162_rn(Biased<CT>::kOffset));
+    a = *reinterpret_cast<const uint32_t*>(&h);
+  }
+  return a;
+}
 
 // One 16-step with biased operands (same fragment roles as w4_step).
 template <typename CT, int NTOK, bool kSplitX>
@@ -106,10 +117,10 @@ __device__ __forceinline__ void w4_step_biased(float (&acc)[NTOK][8][4], float (
 #pragma unroll
     for (int bi = 0; bi < 4; ++bi) {
       const uint32_t sel = (uint32_t)bi | ((uint32_t)bi << 4) | ((uint32_t)(4 + bi) << 8) | ((uint32_t)(4 + bi) << 12);
-      const uint32_t a0 = Biased<CT>::pick(u0, u0s, sel, mask, magic);
-      const uint32_t a1 = Biased<CT>::pick(v0, v0s, sel, mask, magic);
-      const uint32_t a2 = Biased<CT>::pick(u1, u1s, sel, mask, magic);
-      const uint32_t a3 = Biased<CT>::pick(v1, v1s, sel, mask, magic);
+      const uint32_t a0 = unbiased<CT, kSplitX>(Biased<CT>::pick(u0, u0s, sel, mask, magic));
+      const uint32_t a1 = unbiased<CT, kSplitX>(Biased<CT>::pick(v0, v0s, sel, mask, magic));
+      const uint32_t a2 = unbiased<CT, kSplitX>(Biased<CT>::pick(u1, u1s, sel, mask, magic));
+      const uint32_t a3 = unbiased<CT, kSplitX>(Biased<CT>::pick(v1, v1s, sel, mask, magic));
 #pragma unroll
       for (int t = 0; t < NTOK; ++t) {
         mma_wx<CT>(acc[t][wi * 4 + bi], a0, a1, a2, a3, xb[t]);
@@ -326,7 +337,7 @@ w4_stream_kernel(const __grid_constant__ CUtensorMap wmap, const StreamParams p)
       const int64_t n = (int64_t)cg * WCOLS + c;
       // scale and zero are fetched before the ticket so that their latency overlaps the exchange
       float sc = 0.f, z = 0.f;
-      if (n < p.N) { sc = zs_to_f32<ZST>(p.scale, n); z = zs_to_f32<ZST>(p.zero, n) + Biased<CT>::kOffset; }
+      if (n < p.N) { sc = zs_to_f32<ZST>(p.scale, n); z = zs_to_f32<ZST>(p.zero, n) + (kSplitX ? 0.f : Biased<CT>::kOffset); }
       float v[ROWS], xs[ROWS];
 #pragma unroll
       for (int r = 0; r < ROWS; ++r) {

@@ -489,3 +489,23 @@ def test_transposed_matmul_rows_of_any_length_and_alignment(gg, M, N, dtype, zs,
     bound = {torch.bfloat16: 2.0 ** -8, torch.float32: 0.0}[dtype]
     sums = max(2e-5, N / 8 * 2.0 ** -25)
     assert torch.all((got - want).norm(dim=1) <= bound * want.norm(dim=1) + sums * (parts.norm(dim=1) + (parts - want).norm(dim=1)))
+
+
+@pytest.mark.parametrize('M,K,N', [(8, 8192, 20480), (17, 8192, 20480), (16, 5120, 8192)])
+def test_matmul_fp32_keeps_its_precision_on_long_contractions(gg, M, K, N):
+    """fp32 activations: the planes' 2^-17 (2.2e-6 in the 2-norm) and fp32 sums.  Codes with an
+    offset of 128 lose 4e-6 to 5e-6."""
+    from jax_gptq_b200 import quantized_matmul, QuantizedMatrix
+    g = torch.Generator(device='cuda').manual_seed(M + K + N)
+    packed = torch.randint(0, 256, (K // 2, N), generator=g, device='cuda', dtype=torch.uint8)
+    scale = 0.001 + 0.019 * torch.rand(N, generator=g, device='cuda')
+    zero = torch.randint(0, 16, (N,), generator=g, device='cuda').float()
+    x = torch.randn((M, K), generator=g, device='cuda')
+    got = quantized_matmul(x, QuantizedMatrix(packed, zero, scale))
+    err = ref = 0.0
+    for c in range(0, N, 2048):
+        w = packed[:, c:c + 2048]
+        want = x.double() @ ((torch.stack([w & 15, w >> 4], 1).reshape(K, -1).double() - zero[c:c + 2048].double()) * scale[c:c + 2048].double())
+        err += (got[:, c:c + 2048].double() - want).square().sum().item()
+        ref += want.square().sum().item()
+    assert (err / ref) ** 0.5 <= 3.6e-6
