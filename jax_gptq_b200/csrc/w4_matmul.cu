@@ -346,6 +346,8 @@ static bool w4_streams(int64_t M, int64_t N, int64_t K, int x_dtype) {
 //   pair         see plan_w4_pair.
 // On those 495 products the estimates choose within 0.1 % of the better kernel, 5 % at worst.  Examples, single CTA / pair:
 // 64 rows of f16, 4096 x 4096: 35 / 38 us; 96 rows: 45 / 39; 192 rows, 11008 x 4096: 92 / 99; 160 rows of fp32, 4096 x 11008: 85 / 51.
+// fp32 activations stay where the contraction is split: the tensor core's sums lose bits with their length, which an fp32
+// result shows (K = 8192, 64 rows: relative error 2.5e-6 in slices, 1.5e-5 in one chain).
 // More than 512 rows of 16-bit activations always go to the pairs (2048 rows, 4096 x 11008: 293 / 176).
 // The transposed product takes the pairs whenever they can run.  mma.sync kernel / pairs: 33 rows, 4096 x 4096: 106 / 36 us; few
 // outputs and a long contraction, K x N = 64 x 32000: 1 row 639 / 226, 2048 rows 1135 / 476; 11008 x 256: 23 / 16 and 85 / 46.
@@ -362,7 +364,7 @@ static PairPlan w4_pair_choice(int64_t M, int64_t N, int64_t K, int x_dtype, int
   const double single = up.planes == 2 ? 6.0 + waves * ((0.461 + 0.00056 * up.NT) * up.stages_per_split + 1.4 + 0.061 * up.NT) + 0.062 * exchange * up.NT + 2.0 * rows
                                        : 3.1 + waves * ((0.3943 + 0.0007 * up.NT) * up.stages_per_split + 3.26 + 0.0544 * up.NT) +
                                              0.0598 * exchange * (double)(up.mtiles == 1 ? M : up.NT) + 3.9 * rows;
-  pp.use = pp.us < single;
+  pp.use = pp.us < single && (pp.planes == 1 || up.ksplit == 1);
   return pp;
 }
 

@@ -491,10 +491,10 @@ def test_transposed_matmul_rows_of_any_length_and_alignment(gg, M, N, dtype, zs,
     assert torch.all((got - want).norm(dim=1) <= bound * want.norm(dim=1) + sums * (parts.norm(dim=1) + (parts - want).norm(dim=1)))
 
 
-@pytest.mark.parametrize('M,K,N', [(8, 8192, 20480), (17, 8192, 20480), (16, 5120, 8192)])
+@pytest.mark.parametrize('M,K,N', [(33, 8192, 256), (64, 8192, 256), (64, 4096, 4096), (150, 4096, 256), (8, 8192, 20480), (17, 8192, 20480), (16, 5120, 8192)])
 def test_matmul_fp32_keeps_its_precision_on_long_contractions(gg, M, K, N):
-    """fp32 activations: the planes' 2^-17 (2.2e-6 in the 2-norm) and fp32 sums.  Codes with an
-    offset of 128 lose 4e-6 to 5e-6."""
+    """fp32 activations: the planes' 2^-17 (2.2e-6 in the 2-norm) and sums whose chains are cut.  One chain over 8192 indices loses
+    1.5e-5, codes with an offset of 128 4e-6 to 5e-6."""
     from jax_gptq_b200 import quantized_matmul, QuantizedMatrix
     g = torch.Generator(device='cuda').manual_seed(M + K + N)
     packed = torch.randint(0, 256, (K // 2, N), generator=g, device='cuda', dtype=torch.uint8)
